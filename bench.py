@@ -54,8 +54,58 @@ def mask_fractions(n: int):
     return fz, fxy
 
 
-# algorithmic HBM traffic per launch of each pass, in units of one complex
-# half-spectrum field (n*n*(n/2+1)*16 bytes) and one real field (n^3 * 8)
+# algorithmic HBM traffic of a step's kernels, in units of one complex
+# half-spectrum field (n*n*(n/2+1)*16 bytes) and one real field (n^3 * 8).
+# KERNELS: B y backward, C the z pass, D y forward, X the x pass (E1, E2 and
+# the next stage's A of dns_time_kernels).  N is needed only inside the 2/3
+# rule: C stores kz <= kcut, D and X move the masked part; the stage inputs
+# are stored inside the rule only.
+KERNELS = ("B:y-inverse", "C:z-fused", "D:y-forward", "X:x-update")
+
+
+def kernel_units(n: int):
+    """[stage][kernel] -> (complex fields moved, real fields moved), the x
+    pass of the last stage with the next step's transform (its form in the
+    middle of a dns_step call)."""
+    fz, fxy = mask_fractions(n)
+    m = 3 * fz * fxy * fxy  # a packed triple
+    u = []
+    for s in range(4):
+        # B reads u, dv/dx, v, w, dw/dx; writes u, omega_z, v, (w), dw/dy, dw/dx
+        b = (5 + 5, 0) if s == 0 else (5 + 6, 0)
+        # C reads u, v, (w), dw/dx, dw/dy, omega_z (+ the stale velocity in
+        # stage 0, + its store in stage 3) and writes N for kz <= kcut
+        c = ((5 if s == 0 else 6) + 3 * fz, 3 if s in (0, 3) else 0)
+        d = (3 * fz + 3 * fz * fxy, 0)
+        # X reads N, the state and the stage inputs it needs (stage 3: all
+        # three); writes the next input (stage 3: the state) and 5 fields
+        x = (3 * fz * fxy + 3 + (0, m, m, 3 * m)[s] + (3 if s == 3 else m) + 5, 0)
+        u.append([b, c, d, x])
+    return u
+
+
+def kernel_bytes(n: int, s: int = 8):
+    """Algorithmic bytes of every kernel of every stage, s bytes per real
+    (8: FP64, 4: the mixed path's FP32 storage)."""
+    cf = n * n * (n // 2 + 1) * 2 * s
+    rf = n ** 3 * s
+    return [[uc * cf + ur * rf for (uc, ur) in st] for st in kernel_units(n)]
+
+
+def kernel_times(kms):
+    """[stage][kernel] times from dns_time_kernels' [stage][pass] ones."""
+    x = [kms[s][4] + kms[s][5] + (kms[s + 1][0] if s < 3 else kms[0][0]) for s in range(4)]
+    return [[kms[s][1], kms[s][2], kms[s][3], x[s]] for s in range(4)]
+
+
+def step_bytes(n: int, s: int = 8) -> int:
+    """Algorithmic bytes of one RK4 step of this implementation."""
+    return int(sum(map(sum, kernel_bytes(n, s))))
+
+
+# HBM traffic of a step whose six passes a stage run one kernel each, with an
+# accumulator: the model that the fused x pass is reported against
+# (step_hbm's bytes_one_kernel_per_pass), in the units above
 # [stage][pass] -> (complex fields moved, real fields moved).  N is needed
 # only inside the 2/3 rule: C stores kz <= kcut, D and E1 move the masked
 # part, E2 reads N there only.
@@ -93,11 +143,6 @@ def pass_bytes(n: int, s: int = 8):
     cf = n * n * (n // 2 + 1) * 2 * s
     rf = n ** 3 * s
     return [[uc * cf + ur * rf for (uc, ur) in st] for st in pass_units(n)]
-
-
-def step_bytes(n: int, s: int = 8) -> int:
-    """Algorithmic bytes of one RK4 step of this implementation."""
-    return int(sum(map(sum, pass_bytes(n, s))))
 
 
 def step_bytes_model(n: int, s: int = 8) -> int:
@@ -527,18 +572,21 @@ def main() -> int:
     # -- per-kernel timing for the roofline --
     K = dns_b200.KERNELS_PER_STAGE
     kms = ctx.time_kernels(NU, DT, 3).reshape(4, K)
-    pb = pass_bytes(n)
-    share = kms.sum(axis=0)
-    dom = int(np.argmax(share))
+    pb = kernel_bytes(n)
+    kt = np.array(kernel_times(kms))
+    # stage 3's x pass is timed as two launches (the update, the transform)
+    # that read the state twice
+    pb[3][3] += 3 * n * n * (n // 2 + 1) * 16
+    dom = int(np.argmax(kt.sum(axis=0)))
     dom_bytes = sum(pb[s][dom] for s in range(4)) / 4.0
-    dom_ms = float(kms[:, dom].mean())
+    dom_ms = float(kt[:, dom].mean())
     peak, peak_kind = load_peak()
     achieved = dom_bytes / (dom_ms / 1000.0) / 1e9
     traffic = None
     try:
         with open(TRAFFIC) as f:
             tj = json.load(f)
-        traffic = tj.get(str(n), {}).get(dns_b200.PASS_NAMES[dom])
+        traffic = tj.get(str(n), {}).get(KERNELS[dom])
     except Exception:
         pass
     sbytes = step_bytes(n)
@@ -649,16 +697,17 @@ def main() -> int:
                        "l2": "working set %.2f GB >> 126 MB L2, no flush" % (ctx.info()["device_bytes"] / 1e9)},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": dns_b200.PASS_NAMES[dom], "peak_source": peak_kind,
+                         "kernel": KERNELS[dom], "peak_source": peak_kind,
                          "kernel_ms": dom_ms, "kernel_bytes": dom_bytes},
             "step_hbm": {"algorithmic_bytes": sbytes, "achieved_gbs": sbytes * steps_per_s / 1e9,
                          "frac": sbytes * steps_per_s / (peak * 1e9),
+                         "bytes_one_kernel_per_pass": int(sum(map(sum, pass_bytes(n)))),
                          "model_bytes_216C": step_bytes_model(n),
                          "frac_of_model_roofline": step_bytes_model(n) * steps_per_s / (peak * 1e9)},
             "kernel_ms": {dns_b200.PASS_NAMES[p]: [float(kms[s, p]) for s in range(4)] for p in range(K)},
             "e2e": {"value": e2e, "unit": "steps/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "wall_s": wall},
-            "gpu_launches": dns_b200.KERNELS_PER_STEP * args.steps,
+            "gpu_launches": dns_b200.LAUNCHES_PER_STEP * args.steps + 1,
             "mixed": mixed,
             "ensemble": ens,
             "n512": big,

@@ -22,7 +22,7 @@ INCLUDE = os.path.join(ROOT, "include")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-O3", "-lineinfo", "-std=c++17",
+    "-O3", "-lineinfo", "-std=c++17", "-split-compile=0",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
 ]
 

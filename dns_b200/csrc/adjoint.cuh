@@ -59,6 +59,38 @@ __device__ __forceinline__ void curl_at(const PointK &p, cd u, cd v, cd w, cd &o
   oz = make_double2(-az.y, az.x);
 }
 
+// Input U_s of RK stage s at a point: the state (s == 0), the packed stage
+// input inside the 2/3 rule, the state times lin_coef outside it.
+template <class C>
+struct StageIn {
+  const C *u0, *rk;
+  int s;
+  double nudt;
+  __device__ __forceinline__ C at(const Geo &g, const PointK &p, int f) const {
+    using R = sc<C>;
+    if (s > 0 && p.in) {
+      const int ix = (int)p.kx < 0 ? (int)p.kx + g.mk : (int)p.kx;
+      const int iy = (int)p.ky < 0 ? (int)p.ky + g.mk : (int)p.ky;
+      return rk[(3 * (s - 1) + f) * g.slotc + ((long long)ix * g.mk + iy) * g.mp + p.col];
+    }
+    const C z = u0[f * g.slot + p.o];
+    if (s == 0) return z;
+    const R c = (R)(nudt * p.kk);
+    const R m = s == 1 ? lin_coef<0>(c) : s == 2 ? lin_coef<1>(c) : lin_coef<2>(c);
+    return cmk<C>(fma_rn(m, z.x, z.x), fma_rn(m, z.y, z.y));
+  }
+};
+
+// out = U_s on 3 slots
+template <class C>
+__global__ void k_stage_input(StageIn<C> us, C *__restrict__ out, Geo g) {
+  DNSB_FOR_POINTS(g) {
+    const PointK p = point_k(g, q);
+#pragma unroll
+    for (int f = 0; f < 3; f++) out[f * g.slot + p.o] = us.at(g, p, f);
+  }
+}
+
 // out = curl(in) on 3 slots
 template <class C>
 __global__ void k_curl(const C *__restrict__ in, C *__restrict__ out, Geo g) {
@@ -128,7 +160,7 @@ __global__ void k_adj_cross(const RU *__restrict__ u, const RW *__restrict__ om,
 template <int BS, class C>
 __global__ void __launch_bounds__(BS)
     k_adj_collect(const C *__restrict__ Rw, const C *__restrict__ Ru, C *ldU,
-                  const C *__restrict__ Us, const C *lhat_in, C *lhat_out,
+                  StageIn<C> Us, const C *lhat_in, C *lhat_out,
                   const C *__restrict__ lacc, Geo g, double a, double nu, double dt, double bn,
                   double an, bool next, double4 *__restrict__ partial) {
   DD gn{0.0, 0.0}, unused{0.0, 0.0};
@@ -144,7 +176,7 @@ __global__ void __launch_bounds__(BS)
       const long long o = f * g.slot + p.o;
       cd cf = cxyz[f];
       if (Ru) cf = cadd(cf, to_d(Ru[o]));
-      const cd l = to_d(ldU[o]), u = to_d(Us[o]);
+      const cd l = to_d(ldU[o]), u = to_d(Us.at(g, p, f));
       dotp += l.x * u.x;
       dotp += l.y * u.y;
       const cd lus = make_double2(s * cf.x - c * l.x, s * cf.y - c * l.y);

@@ -5,16 +5,16 @@
 //   spectral slots, each [n][n][nfp] complex (double2 for DNS_PREC_FP64,
 //   float2 for DNS_PREC_MIXED):
 //     0..2   SA   state at the start of a step (U_hat, V_hat, W_hat)
-//     3..5   SB   RK stage input (main.c's U_hat during stages 1-3)
-//     6..8   ACC  RK accumulator (main.c's U_hat1)
-//     9..15  WORK partially transformed fields of a stage (six used; all seven
+//     3..6   RK   inputs U_1, U_2, U_3 of stages 1-3 inside the 2/3 rule, packed
+//            (Geo::slotc; main.c's U_hat during stages 1-3)
+//     7..13  WORK partially transformed fields of a stage (six used; all seven
 //            are the float64 staging area of the FP32 path's host transfers)
-//     16     P    pressure of the last stage
+//     14     P    pressure of the last stage
 //   stale real velocity [3][n^3] (main.c's U, V, W between steps)
 //   twiddles, reduction partials.
-// main.c's U_hat0 is SA itself: stage 0 reads SA and writes SB/ACC, stage 3
-// writes the new state back into SA, so the copies of main.c:334-342 and
-// main.c:415-420 disappear.
+// main.c's U_hat0 is SA itself: stages 0-2 read SA and write U_1..U_3, stage 3
+// forms the new state from all of them in SA, so the copies of
+// main.c:334-342 and main.c:415-420 and the accumulator U_hat1 disappear.
 #include "dns_b200.h"
 #include "adjoint.cuh"
 #include "init.cuh"
@@ -39,10 +39,13 @@ namespace {
 
 thread_local std::string g_last_error;
 
-enum { SLOT_SA = 0, SLOT_SB = 3, SLOT_ACC = 6, SLOT_WORK = 9, SLOT_P = 16, NSLOTS = 17 };
-// per RK stage: A x-inverse, B y-inverse, C z fused, D y-forward,
-// E1 x-forward, E2 pointwise update
-enum { KERNELS_PER_STAGE = 6 };
+enum { SLOT_SA = 0, SLOT_RK = 3, SLOT_WORK = 7, SLOT_P = 14, NSLOTS = 15 };
+// passes of an RK stage, as dns_time_kernels reports them: A x-inverse, B
+// y-inverse, C z fused, D y-forward, E1 x-forward, E2 pointwise update
+enum { PASSES_PER_STAGE = 6 };
+// the launches that run them: B, C, D and X, which is a stage's E1 and E2 and
+// the next stage's A in one kernel
+enum { K_B = 0, K_C = 1, K_D = 2, K_X = 3, KERNELS_PER_STAGE = 4 };
 
 int fail(int code, const char *what, const char *file, int line) {
   char buf[512];
@@ -163,9 +166,11 @@ struct dns_ctx {
   cudaStream_t stream = nullptr;
   double4 *diag_host = nullptr;  // pinned
   bool have_state = false;
-  cudaGraphExec_t graph = nullptr;
+  // one RK4 step from the x-transformed state: `step` ends by transforming
+  // the new state for the next one, `last` with the new state
+  cudaGraphExec_t step = nullptr, last = nullptr;
   double cur_nu = NAN, cur_dt = NAN;
-  int kernels_per_step = 4 * KERNELS_PER_STAGE;
+  int kernels_per_step = 4 * PASSES_PER_STAGE;
 };
 
 struct dns_ens {
@@ -177,7 +182,7 @@ struct dns_ens {
   cudaEvent_t fork = nullptr;
   double4 *diag_host = nullptr;  // pinned [nruns]
   std::vector<char> have_state;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t step = nullptr, last = nullptr;  // as in dns_ctx
   int nruns = 0;
   bool params_set = false;
   // the persistent schedule: one cooperative launch per step
@@ -193,8 +198,9 @@ struct dns_ens {
 
 namespace {
 
-constexpr double RK_A[4] = {1 / 6.0, 1 / 3.0, 1 / 3.0, 1 / 6.0};  // main.c:15
-constexpr double RK_B[3] = {0.5, 0.5, 1.0};                       // main.c:16
+// main.c:15-16 (the forward step has them written out in xstage_body)
+constexpr double RK_A[4] = {1 / 6.0, 1 / 3.0, 1 / 3.0, 1 / 6.0};
+constexpr double RK_B[3] = {0.5, 0.5, 1.0};
 
 ColJobs jobs_empty(int njobs) {
   ColJobs j;
@@ -202,14 +208,6 @@ ColJobs jobs_empty(int njobs) {
     j.in_slot[q] = 0, j.out_slot[q] = -1, j.der_slot[q] = -1, j.add_slot[q] = -1;
   j.njobs = njobs;
   j.masked = 0;
-  return j;
-}
-ColJobs jobs_pass_a(int in0) {
-  ColJobs j = jobs_empty(3);
-  const int w = SLOT_WORK;
-  j.in_slot[0] = in0 + 0; j.out_slot[0] = w + SU;
-  j.in_slot[1] = in0 + 1; j.out_slot[1] = w + SV; j.der_slot[1] = w + SOMZ;  // dv/dx
-  j.in_slot[2] = in0 + 2; j.out_slot[2] = w + SW; j.der_slot[2] = w + SDWDX;
   return j;
 }
 ColJobs jobs_pass_b(bool first) {
@@ -244,6 +242,8 @@ struct Ops {
   static constexpr size_t Z_SMEM = (size_t)(2 * N + ZCfg<N>::LINES * ZCfg<N>::XB) * sizeof(C);
   template <int KIND>
   static constexpr size_t ZS_SMEM = ZC<R, N, KIND>::SMEM;
+  using X = XC<R, N>;
+  static constexpr size_t XS_SMEM = X::SMEM;
   // the z pass can keep its real velocity and vorticity (k_zstage_keep)
   static constexpr bool ZKEEP = ZC<R, N, 1>::S2 || ZC<R, N, 1>::F32;
 
@@ -316,6 +316,12 @@ struct Ops {
       if ((e = allow(k_zstage_keep<R, N, 0>, ZS_SMEM<0>))) return e;
       if ((e = allow(k_zstage_keep<R, N, 1>, ZS_SMEM<1>))) return e;
     }
+    if ((e = allow(k_xstage<R, N, -1, true>, XS_SMEM))) return e;
+    if ((e = allow(k_xstage<R, N, 0, true>, XS_SMEM))) return e;
+    if ((e = allow(k_xstage<R, N, 1, true>, XS_SMEM))) return e;
+    if ((e = allow(k_xstage<R, N, 2, true>, XS_SMEM))) return e;
+    if ((e = allow(k_xstage<R, N, 3, true>, XS_SMEM))) return e;
+    if ((e = allow(k_xstage<R, N, 3, false>, XS_SMEM))) return e;
     if ((e = allow(k_zr2c<R, N>, Z_SMEM))) return e;
     if ((e = allow(k_zc2r<R, N>, Z_SMEM))) return e;
     return cudaSuccess;
@@ -355,8 +361,9 @@ struct Ops {
     rec.pick[AXIS][FWD] = pick;
     return cudaSuccess;
   }
-  // Time every register schedule of the four column passes of an RK stage
-  // (their real job tables, batched over the group's first tune_runs(nruns)
+  // Time every register schedule of the four column passes (y: the job
+  // tables of an RK stage, x: three fields, as the initial transform and the
+  // field reads run them; batched over the group's first tune_runs(nruns)
   // runs, on their work slots, whose contents do not matter to an FFT's
   // timing) and keep the fastest of each; once per process, size and tuning
   // run count.  The group launches with the picks (G.pick).  DNS_B200_TUNE=0 keeps the compiler's schedule,
@@ -394,17 +401,18 @@ struct Ops {
     Group Gt = G;  // the first tune_runs runs
     Gt.nruns = G.tune_runs;
     const int io[3] = {SLOT_WORK + SNX, SLOT_WORK + SNY, SLOT_WORK + SNZ};
-    ColJobs jm = jobs_map(io, io, 3);
+    const ColJobs jx = jobs_map(io, io, 3);
+    ColJobs jm = jx;
     jm.masked = 1;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     if (e == cudaSuccess)
-      e = time_cands<0, false>(Gt, st, jobs_pass_a(SLOT_WORK), e0, e1, force, fm[0], rec);
+      e = time_cands<0, false>(Gt, st, jx, e0, e1, force, fm[0], rec);
     if (e == cudaSuccess)
       e = time_cands<1, false>(Gt, st, jobs_pass_b(false), e0, e1, force, fm[2], rec);
     if (e == cudaSuccess) e = time_cands<1, true>(Gt, st, jm, e0, e1, force, fm[3], rec);
-    if (e == cudaSuccess) e = time_cands<0, true>(Gt, st, jm, e0, e1, force, fm[1], rec);
+    if (e == cudaSuccess) e = time_cands<0, true>(Gt, st, jx, e0, e1, force, fm[1], rec);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (e == cudaSuccess) tune_cache[G.tune_runs] = rec;
@@ -468,11 +476,9 @@ struct Ops {
   template <int AXIS, bool FWD>
   static void colpass_io(const Group &G, cudaStream_t st, const C *in, C *out, const ColJobs &jobs,
                          int nruns) {
-    // a masked pass covers the tiles holding kz <= kcut and, along x, the
-    // ky rows with |ky| <= kcut (kernels.cuh maps them back)
+    // a masked pass covers the tiles holding kz <= kcut
     const int tiles = jobs.masked ? G.g.kcut / CW<AXIS> + 1 : G.g.nfp / CW<AXIS>;
-    const int rows = (jobs.masked && AXIS == 0) ? 2 * G.g.kcut + 1 : N;
-    dim3 grid(tiles, rows, jobs.njobs * nruns);
+    dim3 grid(tiles, N, jobs.njobs * nruns);
     colkern<AXIS, FWD>(G)<<<grid, CT<AXIS>, COL_SMEM<AXIS>, st>>>(in, out, tw(G), G.g, jobs);
   }
   template <int AXIS, bool FWD>
@@ -486,41 +492,41 @@ struct Ops {
     return dim3((N * N + ZC<R, N, KIND>::LINES - 1) / ZC<R, N, KIND>::LINES, nruns);
   }
 
-  // Pass `k` (0..KERNELS_PER_STAGE-1) of RK stage `s` for all runs of G:
-  // what it runs, its job table or stage arguments, and its work items (the
-  // launch grid, threads and shared memory of one block).  The standalone
-  // launches (stage_kernel) and the persistent ensemble kernel's plan are
-  // both made from it.
+  static XArgs<R> xargs(const Group &G, int s) {
+    return XArgs<R>{slot(G, SLOT_SA), slot(G, SLOT_RK), slot(G, SLOT_WORK),
+                    (s == 3 && (G.flags & DNS_FLAG_PRESSURE)) ? slot(G, SLOT_P) : nullptr, G.coef};
+  }
+  static dim3 xgrid(const Group &G) { return dim3((G.g.nf + X::W - 1) / X::W, N, G.nruns); }
+
+  // Kernel `k` (K_B..K_X) of RK stage `s` for all runs of G, or with s < 0
+  // the x transform of the state a step starts from: what it runs, its job
+  // table or arguments, and its work items (the launch grid, threads and
+  // shared memory of one block).  The standalone launches (stage_kernel) and
+  // the persistent ensemble kernel's plan are both made from it.
   static PPhase<R> describe(const Group &G, int s, int k) {
     const Geo &g = G.g;
     PPhase<R> P{};
     P.gz = 1;
-    if (k == 0 || k == 1 || k == 3 || k == 4) {
+    if (k == K_B || k == K_D) {
       P.kind = PK_COL;
-      P.axis = (k == 0 || k == 4) ? 0 : 1;
-      P.fwd = k >= 3;
-      if (k == 0) {
-        P.jobs = jobs_pass_a(s == 0 ? SLOT_SA : SLOT_SB);
-      } else if (k == 1) {
+      P.fwd = k == K_D;
+      if (k == K_B) {
         P.jobs = jobs_pass_b(s == 0);
       } else {
-        // D: y forward, E1: x forward (in place on the three N slots); only
-        // the modes inside the 2/3 rule are computed and stored
+        // y forward, in place on the three N slots; only the modes inside
+        // the 2/3 rule are computed and stored
         const int io[3] = {SLOT_WORK + SNX, SLOT_WORK + SNY, SLOT_WORK + SNZ};
         P.jobs = jobs_map(io, io, 3);
         P.jobs.masked = 1;
       }
-      constexpr int cw0 = CW<0>, cw1 = CW<1>, ct0 = CT<0>, ct1 = CT<1>;
-      constexpr int sm0 = (int)COL_SMEM<0>, sm1 = (int)COL_SMEM<1>;
-      const int cw = P.axis == 0 ? cw0 : cw1;
-      // a masked pass covers the tiles holding kz <= kcut and, along x, the
-      // ky rows with |ky| <= kcut (kernels.cuh maps them back)
+      // a masked pass covers the tiles holding kz <= kcut
+      constexpr int cw = CW<1>;
       P.gx = P.jobs.masked ? g.kcut / cw + 1 : g.nfp / cw;
-      P.gy = (P.jobs.masked && P.axis == 0) ? 2 * g.kcut + 1 : N;
+      P.gy = N;
       P.gz = P.jobs.njobs * G.nruns;
-      P.tpi = P.axis == 0 ? ct0 : ct1;
-      P.smem = P.axis == 0 ? sm0 : sm1;
-    } else if (k == 2) {
+      P.tpi = CT<1>;
+      P.smem = (int)COL_SMEM<1>;
+    } else if (k == K_C) {
       P.kind = PK_Z;
       P.sub = s == 0 ? 0 : s < 3 ? 1 : 2;
       const int lines = P.sub == 0 ? ZC<R, N, 0>::LINES : P.sub == 1 ? ZC<R, N, 1>::LINES
@@ -530,53 +536,57 @@ struct Ops {
       P.tpi = ZC<R, N, 0>::THREADS;
       P.smem = (int)(P.sub == 0 ? ZS_SMEM<0> : P.sub == 1 ? ZS_SMEM<1> : ZS_SMEM<2>);
     } else {
-      P.kind = PK_UPD;
+      P.kind = PK_X;
       P.sub = s;
-      StageArgs<R> &sa = P.sa;
-      sa.u0 = slot(G, SLOT_SA);
-      sa.us = slot(G, s == 0 ? SLOT_SA : SLOT_SB);
-      sa.acc = slot(G, SLOT_ACC);
-      sa.next = slot(G, SLOT_SB);
-      sa.ph = (s == 3 && (G.flags & DNS_FLAG_PRESSURE)) ? slot(G, SLOT_P) : nullptr;
-      sa.coef = G.coef;
-      sa.a = RK_A[s];
-      sa.b = s < 3 ? RK_B[s] : 0.0;
-      const long long npad = (long long)N * N * g.nfp;
-      const int per = UPD_THREADS * UpdVec<R>::VP;
-      P.gx = (int)((npad + per - 1) / per);
-      P.gy = G.nruns;
-      P.tpi = UPD_THREADS;
-      P.smem = 0;
+      P.xa = xargs(G, s);
+      const dim3 grid = xgrid(G);
+      P.gx = grid.x;
+      P.gy = grid.y;
+      P.gz = grid.z;
+      P.tpi = X::THREADS;
+      P.smem = (int)XS_SMEM;
     }
     return P;
   }
 
-  // kernel `k` (0..KERNELS_PER_STAGE-1) of RK stage `s`, all runs of G
-  static void stage_kernel(const Group &G, cudaStream_t st, int s, int k) {
+  template <int ST, bool TAIL>
+  static void xpass(const Group &G, cudaStream_t st) {
+    k_xstage<R, N, ST, TAIL>
+        <<<xgrid(G), X::THREADS, XS_SMEM, st>>>(xargs(G, ST), tw(G), G.g);
+  }
+
+  // kernel `k` (K_B..K_X) of RK stage `s`, all runs of G; `tail`: the last
+  // stage's x pass also transforms the new state for the next step
+  static void stage_kernel(const Group &G, cudaStream_t st, int s, int k, bool tail) {
     const Geo &g = G.g;
     C *work = slot(G, SLOT_WORK);
     R *stale = (R *)G.stale;
     const R invn3 = (R)(1.0 / (double)g.nreal);
-    const PPhase<R> P = describe(G, s, k);
-    const dim3 grid(P.gx, P.gy, P.gz);
-    if (P.kind == PK_COL) {
-      ColFn f = P.axis == 0 ? (P.fwd ? colkern<0, true>(G) : colkern<0, false>(G))
-                            : (P.fwd ? colkern<1, true>(G) : colkern<1, false>(G));
-      f<<<grid, P.tpi, P.smem, st>>>((C *)G.S, (C *)G.S, tw(G), g, P.jobs);
-    } else if (P.kind == PK_Z) {
-      if (P.sub == 0)
-        zpass<0>(G, st, work, stale, invn3);
-      else if (P.sub == 1)
-        zpass<1>(G, st, work, stale, invn3);
+    if (k == K_X) {
+      if (s < 0)
+        xpass<-1, true>(G, st);
+      else if (s == 0)
+        xpass<0, true>(G, st);
+      else if (s == 1)
+        xpass<1, true>(G, st);
+      else if (s == 2)
+        xpass<2, true>(G, st);
+      else if (tail)
+        xpass<3, true>(G, st);
       else
-        zpass<2>(G, st, work, stale, invn3);
+        xpass<3, false>(G, st);
+      return;
+    }
+    const PPhase<R> P = describe(G, s, k);
+    if (P.kind == PK_COL) {
+      ColFn f = P.fwd ? colkern<1, true>(G) : colkern<1, false>(G);
+      f<<<dim3(P.gx, P.gy, P.gz), P.tpi, P.smem, st>>>((C *)G.S, (C *)G.S, tw(G), g, P.jobs);
+    } else if (P.sub == 0) {
+      zpass<0>(G, st, work, stale, invn3);
+    } else if (P.sub == 1) {
+      zpass<1>(G, st, work, stale, invn3);
     } else {
-      switch (s) {
-        case 0: k_update<R, N, 0><<<grid, UPD_THREADS, 0, st>>>(work, g, P.sa); break;
-        case 1: k_update<R, N, 1><<<grid, UPD_THREADS, 0, st>>>(work, g, P.sa); break;
-        case 2: k_update<R, N, 2><<<grid, UPD_THREADS, 0, st>>>(work, g, P.sa); break;
-        default: k_update<R, N, 3><<<grid, UPD_THREADS, 0, st>>>(work, g, P.sa); break;
-      }
+      zpass<2>(G, st, work, stale, invn3);
     }
   }
 
@@ -589,13 +599,17 @@ struct Ops {
     pg.stale = (R *)G.stale;
     pg.tw = tw(G);
     pg.invn3 = (R)(1.0 / (double)G.g.nreal);
+    pg.ph[0] = describe(G, -1, K_X);
     for (int s = 0; s < 4; s++)
-      for (int k = 0; k < KERNELS_PER_STAGE; k++) pg.ph[s * KERNELS_PER_STAGE + k] = describe(G, s, k);
+      for (int k = 0; k < KERNELS_PER_STAGE; k++)
+        pg.ph[1 + s * KERNELS_PER_STAGE + k] = describe(G, s, k);
   }
 
-  static void step(const Group &G, cudaStream_t st) {
+  // the x transform of the state, which a step starts from
+  static void first(const Group &G, cudaStream_t st) { stage_kernel(G, st, -1, K_X, true); }
+  static void step(const Group &G, cudaStream_t st, bool tail) {
     for (int s = 0; s < 4; s++)
-      for (int k = 0; k < KERNELS_PER_STAGE; k++) stage_kernel(G, st, s, k);
+      for (int k = 0; k < KERNELS_PER_STAGE; k++) stage_kernel(G, st, s, k, tail);
   }
 
   // forward transform of the three stale real slots into SA (one run)
@@ -737,6 +751,12 @@ int group_init(Group &G, long n, int precision, unsigned flags, int nruns, cudaS
   int kcut = -1;
   while ((double)(kcut + 1) < kmax) kcut++;
   g.kcut = kcut;
+  // packed stage inputs: rows on the slots' pitch granularity where nine
+  // packed fields then fit the four RK slots (all but n = 8)
+  g.mk = 2 * kcut + 1;
+  g.mp = (kcut + W) / W * W;
+  if (9LL * g.mk * g.mk * g.mp > (SLOT_WORK - SLOT_RK) * g.slot) g.mp = kcut + 1;
+  g.slotc = (long long)g.mk * g.mk * g.mp;
   const long long npts = (long long)n * n * g.nf;
   G.diag_blocks = (int)((npts + 255) / 256 < 1184 ? (npts + 255) / 256 : 1184);
 
@@ -945,17 +965,17 @@ int set_coef(const Group &G, cudaStream_t st, const double *nu, const double *dt
 // (U_hat, stale velocity) follow a binomial split of the step range.
 // ---------------------------------------------------------------------------
 // spectral work triples (in units of slots)
-// (the stage inputs U_1..U_3; two buffers for lambda of the step state, one
-// holding the step output's, the other accumulating the step input's, which
-// swap roles after every reversed step; lambda of dU_s; two transform triples)
-enum { X_US1 = 0, X_LA = 9, X_LB = 12, X_LDU = 15, X_T1 = 18, X_T2 = 21, NX = 24 };
+// (two buffers for lambda of the step state, one holding the step output's,
+// the other accumulating the step input's, which swap roles after every
+// reversed step; lambda of dU_s; two transform triples)
+enum { X_LA = 0, X_LB = 3, X_LDU = 6, X_T1 = 9, X_T2 = 12, NX = 15 };
 // real work triples (in units of n^3 fields)
 enum { RE_U = 0, RE_OM = 3, RE_LN = 6, RE_LU = 9, RE_LOM = 12, RE_LSTALE = 15, NRE = 18 };
 
 struct Adj {
   Group G;
   cudaStream_t st = nullptr;
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr, last = nullptr;  // dns_ctx's step and last
   char *arena = nullptr;
   void *sp = nullptr;        // [NX][slot], storage complex type
   double *re = nullptr;      // [NRE][n^3] float64; LU, LOM hold the storage real type
@@ -984,16 +1004,13 @@ template <class R, int N>
 struct AdjOps {
   using O = Ops<R, N>;
   using C = cx<R>;
-  static int copy3(Adj &A, void *dst, const void *src, size_t bytes) {
-    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, A.st));
-    return DNS_OK;
-  }
   static unsigned pblocks(const Adj &A) { return (unsigned)A.nblocks; }
 
-  // U_s: the step input (slot SA, untouched by the forward stages 0-2) or a
-  // kept stage input
-  static const C *stage_input(const Adj &A, int s) {
-    return s == 0 ? (const C *)A.G.slot_ptr(0, SLOT_SA) : A.X<C>(X_US1 + 3 * (s - 1));
+  // U_s: the step input (slot SA, untouched by the forward stages 0-2) and
+  // the packed stage inputs
+  static StageIn<C> stage_input(const Adj &A, int s) {
+    return StageIn<C>{(const C *)A.G.slot_ptr(0, SLOT_SA), (const C *)A.G.slot_ptr(0, SLOT_RK), s,
+                      A.nu * A.dt};
   }
 
   // adjoint of RK stage s: from lambda_dU (X_LDU) and U_s, add lambda_{U_s}
@@ -1004,11 +1021,12 @@ struct AdjOps {
     const Geo &g = G.g;
     const double a = 1.0 / (double)g.nreal;
     const int t3[3] = {0, 1, 2};
-    const C *Us = stage_input(A, s);
+    const StageIn<C> Us = stage_input(A, s);
     const unsigned pb = pblocks(A);
     if constexpr (!O::ZKEEP) {  // the velocity and vorticity of the stage, again
-      if (s > 0) O::c2r_fields(G, A.st, Us, t3, 3, A.Rf(RE_U), a);
-      k_curl<C><<<pb, 256, 0, A.st>>>(Us, A.X<C>(X_T1), g);
+      k_stage_input<C><<<pb, 256, 0, A.st>>>(Us, A.X<C>(X_T2), g);
+      if (s > 0) O::c2r_fields(G, A.st, A.X<C>(X_T2), t3, 3, A.Rf(RE_U), a);
+      k_curl<C><<<pb, 256, 0, A.st>>>(A.X<C>(X_T2), A.X<C>(X_T1), g);
       O::c2r_fields(G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_OM), a);
     }
     k_adj_lamN<C><<<pb, 256, 0, A.st>>>(A.X<C>(X_LDU), A.X<C>(X_T1), g, A.dt);
@@ -1047,23 +1065,22 @@ struct AdjOps {
   // to recover the stage inputs U_1..U_3 (stage 3's output is not needed);
   // the step's state (SA, stale) is left in place for stage 0's adjoint.
   // Where the z pass can keep its real velocity and vorticity, every stage's
-  // z pass (stage 3's too, after its A and B passes; without its stale
-  // store) keeps them for the transposed stage.
+  // z pass (stage 3's too, after its y pass; without its stale store) keeps
+  // them for the transposed stage.
   static int step(Adj &A) {
     const Group &G = A.G;
     const Geo &g = G.g;
     int r;
+    O::first(G, A.st);
     for (int s = 0; s < 4; s++) {
       if (!O::ZKEEP && s == 3) break;
       for (int k = 0; k < KERNELS_PER_STAGE; k++) {
-        if (s == 3 && k > 2) break;
-        if (O::ZKEEP && k == 2)
+        if (s == 3 && k > K_C) break;
+        if (O::ZKEEP && k == K_C)
           O::zpass_keep(G, A.st, s, A.K<R>(s, 0));
         else
-          O::stage_kernel(G, A.st, s, k);
+          O::stage_kernel(G, A.st, s, k, true);
       }
-      if (s < 3 && (r = copy3(A, A.X<C>(X_US1 + 3 * s), G.slot_ptr(0, SLOT_SB), A.slot3())))
-        return r;
     }
     const int lo = A.lhat, li = A.lhat == X_LA ? X_LB : X_LA;
     const C *lacc = A.X<C>(lo);  // lambda of the accumulator: that of the step output
@@ -1094,7 +1111,11 @@ int adj_snap_restore(Adj &A, int k) {
   return DNS_OK;
 }
 int adj_advance(Adj &A, long m) {
-  for (long q = 0; q < m; q++) CK(cudaGraphLaunch(A.graph, A.st));
+  if (m <= 0) return DNS_OK;
+  dispatch(A.G, [&](auto ops) { decltype(ops)::first(A.G, A.st); });
+  CKL();
+  for (long q = 1; q < m; q++) CK(cudaGraphLaunch(A.graph, A.st));
+  CK(cudaGraphLaunch(A.last, A.st));
   return DNS_OK;
 }
 int adj_step_one(Adj &A) {
@@ -1199,16 +1220,19 @@ int adj_reverse(Ex &x, long a, long b, int ka, int free, bool stored) {
   return adj_reverse(x, a, m, ka, free, false);
 }
 
-int ctx_build_graph(dns_ctx *c) {
-  if (c->graph) return DNS_OK;
-  cudaGraph_t gr;
-  CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  dispatch(c->grp, [&](auto ops) { decltype(ops)::step(c->grp, c->stream); });
+// graph of one RK4 step of a group (Ops::step) recorded on `st`
+int group_build_graph(const Group &G, cudaStream_t st, bool tail, cudaGraphExec_t *out) {
+  if (*out) return DNS_OK;
+  cudaGraph_t gr = nullptr;
+  CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+  dispatch(G, [&](auto ops) { decltype(ops)::step(G, st, tail); });
   cudaError_t le = cudaGetLastError();
-  cudaError_t ce = cudaStreamEndCapture(c->stream, &gr);
-  if (le != cudaSuccess) return fail(DNS_ERR_CUDA, cudaGetErrorString(le), __FILE__, __LINE__);
-  CK(ce);
-  cudaError_t ie = cudaGraphInstantiate(&c->graph, gr, 0);
+  cudaError_t ce = cudaStreamEndCapture(st, &gr);
+  if (le != cudaSuccess || ce != cudaSuccess) {
+    if (gr) cudaGraphDestroy(gr);
+    return fail(DNS_ERR_CUDA, cudaGetErrorString(le != cudaSuccess ? le : ce), __FILE__, __LINE__);
+  }
+  cudaError_t ie = cudaGraphInstantiate(out, gr, 0);
   cudaGraphDestroy(gr);
   CK(ie);
   return DNS_OK;
@@ -1258,7 +1282,8 @@ int dns_create(long n, int precision, unsigned flags, dns_ctx **out) {
 int dns_destroy(dns_ctx *c) {
   if (!c) return DNS_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->graph) cudaGraphExecDestroy(c->graph);
+  if (c->step) cudaGraphExecDestroy(c->step);
+  if (c->last) cudaGraphExecDestroy(c->last);
   group_free(c->grp);
   if (c->diag_host) cudaFreeHost(c->diag_host);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1283,9 +1308,13 @@ int dns_step(dns_ctx *c, double nu, double dt, long nsteps) {
     c->cur_nu = nu;
     c->cur_dt = dt;
   }
-  int st = ctx_build_graph(c);
+  int st = group_build_graph(c->grp, c->stream, false, &c->last);
+  if (st == DNS_OK && nsteps > 1) st = group_build_graph(c->grp, c->stream, true, &c->step);
   if (st != DNS_OK) return st;
-  for (long s = 0; s < nsteps; s++) CK(cudaGraphLaunch(c->graph, c->stream));
+  dispatch(c->grp, [&](auto ops) { decltype(ops)::first(c->grp, c->stream); });
+  CKL();
+  for (long s = 1; s < nsteps; s++) CK(cudaGraphLaunch(c->step, c->stream));
+  CK(cudaGraphLaunch(c->last, c->stream));
   return DNS_OK;
 }
 
@@ -1413,7 +1442,8 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
     c->cur_nu = nu;
     c->cur_dt = dt;
   }
-  const int K = c->kernels_per_step;
+  // launches of a step: the x transform of the state, then B, C, D, X a stage
+  const int K = c->kernels_per_step, L = 1 + 4 * KERNELS_PER_STAGE;
   // destroyed on every return path, the early ones of CK included
   struct Events {
     std::vector<cudaEvent_t> v;
@@ -1422,25 +1452,41 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
         if (e) cudaEventDestroy(e);
     }
   } evs;
-  evs.v.assign(K + 1, nullptr);
+  evs.v.assign(L + 1, nullptr);
   std::vector<cudaEvent_t> &ev = evs.v;
   for (auto &e : ev) CK(cudaEventCreate(&e));
   for (int k = 0; k < K; k++) ms[k] = 0.0;
   int st = DNS_OK;
   for (long s = 0; s < nsteps && st == DNS_OK; s++) {
     CK(cudaEventRecord(ev[0], c->stream));
-    for (int k = 0; k < K; k++) {
+    for (int k = 0; k < L; k++) {
+      const int q = k - 1;
       dispatch(c->grp, [&](auto ops) {
-        decltype(ops)::stage_kernel(c->grp, c->stream, k / KERNELS_PER_STAGE, k % KERNELS_PER_STAGE);
+        decltype(ops)::stage_kernel(c->grp, c->stream, k == 0 ? -1 : q / KERNELS_PER_STAGE,
+                                    k == 0 ? (int)K_X : q % KERNELS_PER_STAGE, false);
       });
       CK(cudaEventRecord(ev[k + 1], c->stream));
     }
     st = check_launch(__FILE__, __LINE__);
-    CK(cudaEventSynchronize(ev[K]));
-    for (int k = 0; k < K; k++) {
+    CK(cudaEventSynchronize(ev[L]));
+    for (int k = 0; k < L; k++) {
       float t = 0.f;
       CK(cudaEventElapsedTime(&t, ev[k], ev[k + 1]));
-      ms[k] += t;
+      if (k == 0) {
+        ms[0] += t;
+        continue;
+      }
+      double *row = ms + (k - 1) / KERNELS_PER_STAGE * PASSES_PER_STAGE;
+      const int kern = (k - 1) % KERNELS_PER_STAGE;
+      if (kern != K_X) {
+        row[1 + kern] += t;
+      } else {  // E1 and E2 of this stage and, except after the last, A of the next
+        const bool tail = k + 1 < L;
+        const double share = t / (tail ? 3.0 : 2.0);
+        row[4] += share;
+        row[5] += share;
+        if (tail) row[PASSES_PER_STAGE] += share;
+      }
     }
   }
   for (int k = 0; k < K; k++) ms[k] /= (double)nsteps;
@@ -1451,7 +1497,8 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
 /* ensemble                                                            */
 /* ------------------------------------------------------------------ */
 
-static int ens_build_graph(dns_ens *e);
+static int ens_build_graph(dns_ens *e, bool tail, cudaGraphExec_t *out);
+static int ens_step_batched(dns_ens *e, long nsteps);
 extern "C++" {
 // ---- the persistent schedule ----
 static bool ens_persistent_supported(const dns_ens *e) {
@@ -1552,7 +1599,7 @@ static int ens_time_steps(dns_ens *e, float *ms) {
   int st = ce == cudaSuccess ? DNS_OK : fail(DNS_ERR_CUDA, cudaGetErrorString(ce), __FILE__, __LINE__);
   auto one = [&]() -> int {
     if (e->mode == 1) return ens_step_persistent(e, 1);
-    CK(cudaGraphLaunch(e->graph, e->stream));
+    CK(cudaGraphLaunch(e->step, e->stream));  // a step in the middle of a call
     return DNS_OK;
   };
   if (st == DNS_OK) st = one();
@@ -1583,7 +1630,8 @@ static int ens_choose_schedule(dns_ens *e, unsigned flags) {
   const bool want_p = can && !(flags & DNS_FLAG_ENS_BATCHED);
   if (want_b) {
     e->mode = 0;
-    st = ens_build_graph(e);
+    st = ens_build_graph(e, true, &e->step);
+    if (st == DNS_OK) st = ens_build_graph(e, false, &e->last);
     if (st == DNS_OK && want_p) st = ens_time_steps(e, &e->step_ms[0]);
   }
   if (st == DNS_OK && want_p) {
@@ -1600,7 +1648,8 @@ static int ens_choose_schedule(dns_ens *e, unsigned flags) {
 int dns_ens_destroy(dns_ens *e) {
   if (!e) return DNS_OK;
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->graph) cudaGraphExecDestroy(e->graph);
+  if (e->step) cudaGraphExecDestroy(e->step);
+  if (e->last) cudaGraphExecDestroy(e->last);
   if (e->pgraph) cudaGraphExecDestroy(e->pgraph);
   if (e->pplan) cudaFree(e->pplan);
   if (e->psync) cudaFree(e->psync);
@@ -1710,17 +1759,17 @@ int dns_ens_set_params(dns_ens *e, const double *nu, const double *dt) {
   return DNS_OK;
 }
 
-// one graph: a fork per size group (its own stream), each group's 24
+// one graph: a fork per size group (its own stream), each group's 16
 // batched kernels, then a join
-static int ens_build_graph(dns_ens *e) {
-  if (e->graph) return DNS_OK;
+static int ens_build_graph(dns_ens *e, bool tail, cudaGraphExec_t *out) {
+  if (*out) return DNS_OK;
   cudaGraph_t gr;
   CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
   cudaEventRecord(e->fork, e->stream);
   for (size_t q = 0; q < e->groups.size(); q++) {
     cudaStreamWaitEvent(e->gstreams[q], e->fork, 0);
     const Group &G = e->groups[q];
-    dispatch(G, [&](auto ops) { decltype(ops)::step(G, e->gstreams[q]); });
+    dispatch(G, [&](auto ops) { decltype(ops)::step(G, e->gstreams[q], tail); });
     cudaEventRecord(e->gevents[q], e->gstreams[q]);
     cudaStreamWaitEvent(e->stream, e->gevents[q], 0);
   }
@@ -1728,9 +1777,18 @@ static int ens_build_graph(dns_ens *e) {
   cudaError_t ce = cudaStreamEndCapture(e->stream, &gr);
   if (le != cudaSuccess) return fail(DNS_ERR_CUDA, cudaGetErrorString(le), __FILE__, __LINE__);
   CK(ce);
-  cudaError_t ie = cudaGraphInstantiate(&e->graph, gr, 0);
+  cudaError_t ie = cudaGraphInstantiate(out, gr, 0);
   cudaGraphDestroy(gr);
   CK(ie);
+  return DNS_OK;
+}
+
+static int ens_step_batched(dns_ens *e, long nsteps) {
+  for (const Group &G : e->groups)
+    dispatch(G, [&](auto ops) { decltype(ops)::first(G, e->stream); });
+  CKL();
+  for (long s = 1; s < nsteps; s++) CK(cudaGraphLaunch(e->step, e->stream));
+  CK(cudaGraphLaunch(e->last, e->stream));
   return DNS_OK;
 }
 
@@ -1740,11 +1798,7 @@ int dns_ens_step(dns_ens *e, long nsteps) {
     if (!e->have_state[r]) return fail(DNS_ERR_STATE, "a run has no velocity", __FILE__, __LINE__);
   if (!e->params_set) return fail(DNS_ERR_STATE, "nu and dt not set", __FILE__, __LINE__);
   if (nsteps == 0) return DNS_OK;
-  if (e->mode == 1) return ens_step_persistent(e, nsteps);
-  int st = ens_build_graph(e);
-  if (st != DNS_OK) return st;
-  for (long s = 0; s < nsteps; s++) CK(cudaGraphLaunch(e->graph, e->stream));
-  return DNS_OK;
+  return e->mode == 1 ? ens_step_persistent(e, nsteps) : ens_step_batched(e, nsteps);
 }
 
 int dns_ens_get_schedule(dns_ens *e, char *buf, long len) {
@@ -1848,6 +1902,7 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
   auto cleanup = [&]() {
     if (A.st) cudaStreamSynchronize(A.st);
     if (A.graph) cudaGraphExecDestroy(A.graph);
+    if (A.last) cudaGraphExecDestroy(A.last);
     if (A.arena) cudaFree(A.arena);
     group_free(A.G);
     if (A.st) cudaStreamDestroy(A.st);
@@ -1890,19 +1945,8 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
       if (e != cudaSuccess) r = fail(DNS_ERR_CUDA, cudaGetErrorString(e), __FILE__, __LINE__);
     }
   }
-  if (r == DNS_OK) {  // graph of one forward step
-    cudaGraph_t gr;
-    cudaError_t e = cudaStreamBeginCapture(A.st, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-      dispatch(A.G, [&](auto ops) { decltype(ops)::step(A.G, A.st); });
-      e = cudaStreamEndCapture(A.st, &gr);
-      if (e == cudaSuccess) {
-        e = cudaGraphInstantiate(&A.graph, gr, 0);
-        cudaGraphDestroy(gr);
-      }
-    }
-    if (e != cudaSuccess) r = fail(DNS_ERR_CUDA, cudaGetErrorString(e), __FILE__, __LINE__);
-  }
+  if (r == DNS_OK) r = group_build_graph(A.G, A.st, true, &A.graph);
+  if (r == DNS_OK) r = group_build_graph(A.G, A.st, false, &A.last);
   // J alone: the forward sweep is all it takes (no snapshots are needed
   // beyond the first, and no reverse sweep runs)
   const bool want_grad = gU || gV || gW || gnu;

@@ -17,36 +17,43 @@
 // The same slot shape holds partially transformed data: after the x pass the
 // first index is x instead of kx, after the y pass the second is y.
 //
-// One RK stage = six kernels:
-//   A   x backward  state (3) -> u,v,w and d/dx of v,w            (per field)
+// One RK stage = four kernels:
 //   B   y backward  5 slots -> u,v,w, omega_z = dv/dx - du/dy, dw/dx, dw/dy
 //   C   z pass      per z line: vorticity from the 6 slots, u and omega to
 //                   real space, N = u x omega, N back to z spectral (stored
 //                   for kz <= kcut); real space touches HBM only for the
 //                   stale velocity
 //   D   y forward   3 slots, in place, tiles with kz <= kcut, |ky| <= kcut kept
-//   E1  x forward   3 slots, in place, rows |ky| <= kcut, |kx| <= kcut kept
-//   E2  update      2/3 mask, projection, viscous term, RK4 updates
+//   X   x update    per x line of all three fields: x forward of N, 2/3 mask,
+//                   projection, viscous term and RK4 update, and the x
+//                   backward transforms of the next stage's input: u,v,w and
+//                   d/dx of v,w
+// The first stage of a dns_step call is preceded by X's backward half alone
+// (from the stored state), its last step's last X ends with the update.
 // The vorticity is assembled from spectral derivatives taken on the axis a
-// pass owns (x in A, y in B, z in C), so A, B, D and E1 work on one field per
-// tile and need no cross-field staging.  N only enters the update through
-// the 2/3 rule (main.c:381-386), so C, D and E1 move only those modes and E2
-// reads N there only.
+// pass owns (x in X, y in B, z in C), so B and D work on one field per tile
+// and need no cross-field staging.  N only enters the update through the 2/3
+// rule (main.c:381-386), so C, D and X move only those modes of it.
 #pragma once
 #include "fft_core.cuh"
 
 namespace dnsb {
 
 // work slots of the stage (after pass B, SOMZ holds omega_z = dv/dx - du/dy;
-// after pass A it holds dv/dx).  The z pass writes N = u x omega over the
+// after the x pass it holds dv/dx).  The z pass writes N = u x omega over the
 // slots SNX, SNY, SNZ (those of u, v and dw/dy), each once the line's input
-// in it has been read, and D, E1 and E2 take N from there.
+// in it has been read, and D and X take N from there.
 enum { SU = 0, SV = 1, SDWDY = 2, SOMZ = 3, SDWDX = 4, SW = 5, NWORK = 6 };
 enum { SNX = 0, SNY = 1, SNZ = 2 };
 
 struct Geo {
   int n, nf, nfp;
   int kcut;              // 2/3 rule: a wavenumber is kept iff |k| <= kcut
+  // RK stage inputs are stored inside the 2/3 rule only, packed as
+  // [stage][field][mk: kx][mk: ky][mp: kz] with mk = 2 kcut + 1 rows (index
+  // k for k >= 0, mk + k for k < 0) of pitch mp
+  int mk, mp;
+  long long slotc;       // mk * mk * mp: complex elements per packed field
   long long slot;        // complex elements per spectral slot (n*n*nfp)
   long long nreal;       // n^3
   long long run_spec;    // complex elements between two runs' slot sets
@@ -58,10 +65,9 @@ struct Geo {
 // an output slot and optionally the derivative i*k*f (k along the pass axis)
 // to a der slot, in every run of the batch; with an add slot the derivative
 // output is add - i*k*f instead (the same tile of another slot).  A masked
-// pass (the forward passes of N, whose result only enters the update inside
+// pass (the y forward pass of N, whose result only enters the update inside
 // the 2/3 rule, main.c:381-386) is launched on the column tiles that hold
-// kz <= kcut only, in the x pass also on the ky rows with |ky| <= kcut only,
-// and stores only |k| <= kcut along its own axis.
+// kz <= kcut only and stores only |ky| <= kcut.
 struct ColJobs {
   int in_slot[8];
   int out_slot[8];   // -1: no plain output
@@ -151,10 +157,7 @@ __device__ __forceinline__ void colpass_body(const cx<R> *__restrict__ in, cx<R>
   const int p = b.tid % W, t = b.tid / W;
   const int col = b.x * W + p;
   const bool ok = col < g.nf;
-  // j for the x pass, i for the y pass; a masked x pass is launched on the
-  // 2 kcut + 1 rows with |ky| <= kcut only: rows past kcut map to n - kcut..
-  int fixed = b.y;
-  if (AXIS == 0 && jobs.masked && fixed > g.kcut) fixed += N - (2 * g.kcut + 1);
+  const int fixed = b.y;  // j for the x pass, i for the y pass
   const int job = b.z % jobs.njobs;
   const long long rb = (long long)(b.z / jobs.njobs) * g.run_spec;
   in += rb;
@@ -914,254 +917,356 @@ __global__ void __launch_bounds__(ZC<R, N, KIND>::THREADS, ZC<R, N, KIND>::MINB)
 }
 
 // ---------------------------------------------------------------------------
-// E2: after the x forward transform of the three N slots (E1), the pointwise
-// update of main.c:381-413 on the full half spectrum:
-//   dU  = N * (mask * dt)
-//   P   = kk > 0 ? (dU kx + dV ky + dW kz) / kk : 0
-//   dU -= P kx + nu dt kk U_s          (same for V, W)
-//   ST 0:   next = u0 + b0 dU,  acc = u0 + a0 dU      (u_s == u0)
-//   ST 1,2: next = u0 + b dU,   acc += a dU
-//   ST 3:   u0   = acc + a3 dU   (the state of the next step)
-// A pure streaming kernel, one thread per half-spectrum point (two in FP32).
-// The FP64 path computes in FP64; the mixed path computes in FP32 with the
-// viscous coefficient nu dt |k|^2 formed in FP64 (update_point_f32).
+// X: one block holds the x lines of the three fields over W adjacent kz
+// columns at one ky (N / E * W threads) and takes RK stage ST from N to the
+// next stage's x-transformed fields:
+//   x forward of N (main.c:378-380), inside the 2/3 rule only,
+//   dU  = N * dt,  P = kk > 0 ? (dU kx + dV ky + dW kz) / kk : 0
+//   dU -= P kx + nu dt kk U_s            (same for V, W; main.c:381-413)
+//   ST 0:  U_1 = U_0 + dU / 2     ST 1: U_2 = U_0 + dU / 2
+//   ST 2:  U_3 = U_0 + dU
+//   ST 3:  U_0' = U_3 + ((U_1 - U_0) + 2 (U_2 - U_0) - 2 (U_3 - U_0)) / 3 + dU / 6
+//          (the RK4 sum of main.c:15 written with the stage inputs, which
+//          are kept, in place of an accumulator; the bracket is a sum of
+//          increments, so only the last additions round at |U|)
+//   x backward of the result: u, v, w and i kx v, i kx w  (TAIL; ST < 0: of
+//   the stored state alone)
+// Outside the 2/3 rule N is masked to zero, so the stage inputs there are the
+// state times a polynomial in c = nu dt kk and are formed from the state where
+// they are needed (lin_coef): only the state itself is stored there, by ST 3.
+//
+// The fields go through the block one after another, each thread owning the
+// same points of all three, so that the projection needs no exchange; the
+// transformed N of two fields (then the results that wait for their
+// transform) are held in shared memory, each thread reading back its own.
+//
+// One launch reads N (4/9 of 3 slots), the state (3 slots) and the packed
+// stage inputs, and writes 5 slots and one packed triple: 11.1 slots in a
+// middle stage, where the three kernels it replaces (the x forward pass, the
+// update and the next x backward pass) moved 26.1.  Middle stage, one B200,
+// before (sum of the three) and now: FP64 n = 128 0.098 -> 0.056 ms, n = 256
+// 0.62 -> 0.36 (4.2 TB/s), n = 512 5.24 -> 3.56; FP32 0.070 -> 0.033, 0.345 ->
+// 0.194 (3.9 TB/s), 2.76 -> 1.86.  It is bound by the shared-memory pipe (the
+// exchanges and the waiting fields) and by the loads in flight.
 // ---------------------------------------------------------------------------
-// pointers are those of run 0; run r adds r * run_spec.  coef[2 r] = nu,
-// coef[2 r + 1] = dt of run r (device memory, so a captured graph picks up
-// new values without being rebuilt).
 template <class R>
-struct StageArgs {
-  cx<R> *u0;    // step start state (3 slots); ST 3 writes the new state here
-  cx<R> *us;    // stage input (3 slots)
-  cx<R> *acc;   // RK accumulator (3 slots)
-  cx<R> *next;  // next stage input (3 slots)
+struct XArgs {
+  cx<R> *u0;    // state (3 slots); ST 3 writes the new state here
+  cx<R> *rk;    // packed stage inputs U_1, U_2, U_3 inside the 2/3 rule
+  cx<R> *work;  // work slots
   cx<R> *ph;    // pressure slot or nullptr
-  const double *coef;
-  double a, b;  // RK coefficients of the stage (main.c:15-16)
+  const double *coef;  // coef[2 r] = nu, coef[2 r + 1] = dt of run r (device
+                       // memory, so a captured graph picks up new values)
 };
 
-// Inputs and results of one point.  A thread loads every input of its
-// points before the first store: as far as the compiler knows the stores may
-// alias later inputs, which would otherwise hold loads back behind them.
-template <class R>
-struct UpdIn {
-  cx<R> n[3];   // N slots (E1 output)
-  cx<R> us[3];  // stage input
-  cx<R> z[3];   // u0 (ST 1, 2)
-  cx<R> a[3];   // accumulator (ST 1, 2, 3)
+// Plans of the X pass: 8 values per thread, one exchange more than the
+// column plans at n = 128 and 256, for 12 warps of FP64 (168 registers) and
+// 24 of FP32 (80) beside the buffers (16 values per thread, n = 256 FP64 at 6
+// or 8 warps: middle stage 0.38 ms against 0.36; FP32 0.209 against 0.194).
+template <int L>
+struct XPlan : Plan<L> {};
+template <> struct XPlan<16>  { static constexpr int E = 8, NS = 2, R0 = 8, R1 = 2, R2 = 1, R3 = 1; };
+template <> struct XPlan<128> { static constexpr int E = 8, NS = 3, R0 = 8, R1 = 8, R2 = 2, R3 = 1; };
+template <> struct XPlan<256> { static constexpr int E = 8, NS = 3, R0 = 8, R1 = 8, R2 = 4, R3 = 1; };
+template <> struct XPlan<512> { static constexpr int E = 8, NS = 3, R0 = 8, R1 = 8, R2 = 8, R3 = 1; };
+
+// Tile of the X pass.  Its three buffers (3 N W values) and L1 share the SM's
+// 256 KB, and what is left to L1 bounds the loads in flight: more resident
+// blocks than these measured slower (FP64 n = 256: 3 blocks of 64-byte rows
+// 0.36 ms, 4 blocks 0.42, 2 of 128-byte rows 0.39; FP32 n = 256: 3 blocks of
+// 64-byte rows 0.194, 4 blocks 0.25, 2 of 128-byte rows 0.23).  At n = 512 one
+// block of 128-byte rows beats two of 64-byte rows (FP64 3.56 against 3.90
+// ms, FP32 1.86 against 2.03).
+template <class R, int N>
+struct XC {
+  using P = XPlan<N>;
+  static constexpr int W = sizeof(R) == 8 ? (N == 256 ? 4 : 8) : (N == 512 ? 16 : 8);
+  static constexpr int E = P::E, T = N / E;
+  static constexpr int THREADS = T * W;
+  // twiddle entries (even, so the buffers stay 16-byte aligned)
+  static constexpr int TWN = (StageTw<P>::SIZE + 2) / 2 * 2;
+  // rows shorter than 128 bytes: one row of pad per R0 positions, which the
+  // first exchange writes R0 apart
+  static constexpr int SH = W * sizeof(cx<R>) >= 128 ? 30 : P::R0 == 16 ? 4 : 3;
+  static constexpr int XB = (N + (N >> SH)) * W;  // exchange buffer
+  static constexpr size_t SMEM = (size_t)(TWN + XB + 2 * N * W) * sizeof(cx<R>);
+  static constexpr int WANT = (sizeof(R) == 8 ? 384 : 768) / THREADS;
+  static constexpr int MINB = WANT < 1 ? 1 : WANT > 16 ? 16 : WANT;  // blocks per SM
 };
-template <class R>
-struct UpdOut {
-  cx<R> o1[3];  // next stage input (ST 0-2) or the new state (ST 3)
-  cx<R> o2[3];  // accumulator (ST 0-2)
-  cx<R> p;      // pressure
+template <int W, int SH>
+struct XIdx {
+  int p;
+  __device__ __forceinline__ int operator()(int pos) const { return (pos + (pos >> SH)) * W + p; }
 };
 
-template <class R, int ST>
-__device__ __forceinline__ void update_point(const UpdIn<R> &in, UpdOut<R> &out, const Geo &g,
-                                             const StageArgs<R> &sa, double nu, double dt, int i,
-                                             int j, int col) {
+// The x pass writes its roundings out (no product is left to be contracted
+// into a following addition at the compiler's choice): every kernel that
+// inlines it computes the same bits, and the value it stores is the one it
+// transforms on the spot.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
+
+// Outside the 2/3 rule dU = -c U_s with c = nu dt kk: the stage input that
+// stage ST forms (ST 3: the new state) is U_0 + m U_0 with this m.
+template <int ST, class R>
+__device__ __forceinline__ R lin_coef(R c) {
+  const R h = R(0.5) * c;
+  const R m1 = -h;
+  if (ST == 0) return m1;
+  const R m2 = mul_rn(-h, R(1) + m1);
+  if (ST == 1) return m2;
+  const R m3 = mul_rn(-c, R(1) + m2);
+  if (ST == 2) return m3;
+  return fma_rn(m1 + R(2) * m2 + m3, R(1.0 / 3.0), mul_rn(mul_rn(-c, R(1) + m3), R(1.0 / 6.0)));
+}
+
+// loads that leave no line in L1 (little of it is left beside the buffers,
+// and lines reserved for loads in flight would bound how many there are)
+template <class C>
+__device__ __forceinline__ C ldcg(const C *p) {
+  return __ldcg(p);
+}
+// 16-byte asynchronous copy from global to shared memory, past L1
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+template <class R, int N, int ST, bool TAIL, class Sync>
+__device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__restrict__ twg,
+                                            const Geo &g, const Blk b, Sync sync,
+                                            unsigned char *smem) {
   using C = cx<R>;
-  const int ikx = kwave(i, g.n), iky = kwave(j, g.n);
-  const double kx = (double)ikx, ky = (double)iky, kz = (double)col;
-  const bool inm = (ikx < 0 ? -ikx : ikx) <= g.kcut && (iky < 0 ? -iky : iky) <= g.kcut &&
-                   col <= g.kcut;
-  // main.c multiplies by the 0/1 mask; N is selected instead, because the
-  // forward passes leave the entries outside the 2/3 rule unwritten
-  const double2 zero = make_double2(0.0, 0.0);
-  double2 du = inm ? cscale(to_d(in.n[0]), dt) : zero;
-  double2 dv = inm ? cscale(to_d(in.n[1]), dt) : zero;
-  double2 dw = inm ? cscale(to_d(in.n[2]), dt) : zero;
-  const double kk = kx * kx + ky * ky + kz * kz;
-  double2 P;
-  if (kk > 0) {
-    P.x = (du.x * kx + dv.x * ky + dw.x * kz) / kk;
-    P.y = (du.y * kx + dv.y * ky + dw.y * kz) / kk;
+  using X = XC<R, N>;
+  using P = typename X::P;
+  constexpr int W = X::W, E = X::E, T = X::T, TH = X::THREADS;
+  static_assert(ST >= 0 || TAIL, "the plain backward pass has a tail");
+  C *st = (C *)smem;
+  C *xb = st + X::TWN;
+  const int p = b.tid % W, t = b.tid / W;
+  // own points of the two fields that wait: s0[e * TH], s1[e * TH]
+  C *s0 = xb + X::XB + b.tid, *s1 = s0 + E * TH;
+  const int j = b.y, col = b.x * W + p;
+  const bool ok = col < g.nf;
+  const int iky = kwave(j, N);
+  const bool yin = (iky < 0 ? -iky : iky) <= g.kcut;             // same for the block
+  const bool hasn = ST >= 0 && yin && (int)(b.x * W) <= g.kcut;  // same for the block
+  const bool zin = yin && col <= g.kcut;
+  const long long rb = (long long)b.z * g.run_spec;
+  const unsigned rs = (unsigned)N * g.nfp;
+  const unsigned base = (unsigned)j * g.nfp + col + t * rs;  // of point e = 0
+  C *u0 = a.u0 + rb + base;
+  C *wk = a.work + rb + base;
+  const XIdx<W, X::SH> idx{p};
+  // offset of own point e in a slot, relative to `base`
+  auto at = [&](int e) -> long long { return (long long)((unsigned)(T * e) * rs); };
+  const double nu = ST < 0 ? 0.0 : a.coef[2 * b.z], dt = ST < 0 ? 0.0 : a.coef[2 * b.z + 1];
+  const double nudt = nu * dt;
+  const int kyz = iky * iky + col * col;
+  auto kin = [&](int ik) { return (ik < 0 ? -ik : ik) <= g.kcut; };
+  C v[E];
+
+  // The first inputs: one field to registers, the other two on their way to
+  // their places in shared memory meanwhile (N, or the state where there is
+  // no N).  FP32 copies pairs of columns, the even thread those of s0 and the
+  // odd thread those of s1; a pair's second column may lie past the valid
+  // ones (in the row's padding, or past kcut) and is not used then.
+  const bool first_ok = hasn ? zin : ok;
+  const C *f0 = hasn ? wk + SNX * g.slot : u0;
+  const C *f1 = hasn ? wk + SNY * g.slot : u0 + g.slot;
+  const C *f2 = hasn ? wk + SNZ * g.slot : u0 + 2 * g.slot;
+  if constexpr (sizeof(C) == 16) {
+    if (first_ok) {
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        copy16(s0 + e * TH, f1 + at(e));
+        copy16(s1 + e * TH, f2 + at(e));
+      }
+    }
   } else {
-    P = make_double2(0.0, 0.0);
+    static_assert(W % 2 == 0, "pairs of columns");
+    const int odd = p & 1;
+    if (odd ? (hasn ? col - 1 <= g.kcut : col - 1 < g.nf) : first_ok) {
+      C *d = (odd ? s1 : s0) - odd;
+      const C *s = (odd ? f2 : f1) - odd;
+#pragma unroll
+      for (int e = 0; e < E; e++) copy16(d + e * TH, s + at(e));
+    }
   }
-  const double c = nu * dt * kk;
-  const double2 us0 = to_d(in.us[0]), us1 = to_d(in.us[1]), us2 = to_d(in.us[2]);
-  du = make_double2(du.x - (P.x * kx + c * us0.x), du.y - (P.y * kx + c * us0.y));
-  dv = make_double2(dv.x - (P.x * ky + c * us1.x), dv.y - (P.y * ky + c * us1.y));
-  dw = make_double2(dw.x - (P.x * kz + c * us2.x), dw.y - (P.y * kz + c * us2.y));
-  out.p = from_d<C>(P);
-  auto axpy = [](double2 x, double s, double2 y) {
-    return make_double2(x.x + s * y.x, x.y + s * y.y);
+#pragma unroll
+  for (int e = 0; e < E; e++) v[e] = first_ok ? ldcg(f0 + at(e)) : czero<C>();
+  auto copies_done = [&]() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (sizeof(C) != 16) __syncwarp();
   };
-  const double2 d[3] = {du, dv, dw};
+  auto landed = [&](const C *s, int e) { return first_ok ? s[e * TH] : czero<C>(); };
+  build_stage_tw<N, P>(st, twg, N, b.tid, b.nt);
+  sync();
+
+  if (!hasn) {
+    copies_done();
+    if constexpr (ST >= 0) {
 #pragma unroll
-  for (int f = 0; f < 3; f++) {
-    if (ST == 0) {  // us == u0
-      const double2 u = to_d(in.us[f]);
-      out.o1[f] = from_d<C>(axpy(u, sa.b, d[f]));
-      out.o2[f] = from_d<C>(axpy(u, sa.a, d[f]));
-    } else if (ST < 3) {
-      out.o1[f] = from_d<C>(axpy(to_d(in.z[f]), sa.b, d[f]));
-      out.o2[f] = from_d<C>(axpy(to_d(in.a[f]), sa.a, d[f]));
-    } else {
-      out.o1[f] = from_d<C>(axpy(to_d(in.a[f]), sa.a, d[f]));
+      for (int e = 0; e < E; e++) {
+        const int ik = kwave(t + T * e, N);
+        const R m = lin_coef<ST>((R)(nudt * (double)(ik * ik + kyz)));
+        const C z1 = landed(s0, e), z2 = landed(s1, e);
+        v[e] = cmk<C>(fma_rn(m, v[e].x, v[e].x), fma_rn(m, v[e].y, v[e].y));
+        const C r1 = cmk<C>(fma_rn(m, z1.x, z1.x), fma_rn(m, z1.y, z1.y));
+        const C r2 = cmk<C>(fma_rn(m, z2.x, z2.x), fma_rn(m, z2.y, z2.y));
+        s0[e * TH] = r1;
+        s1[e * TH] = r2;
+        if (ST == 3 && ok) {
+          u0[at(e)] = v[e];
+          u0[at(e) + g.slot] = r1;
+          u0[at(e) + 2 * g.slot] = r2;
+        }
+      }
     }
-  }
-}
-
-// The mixed path's update: FP32 arithmetic for the projection and the RK
-// axpys (the storage precision), FP64 only for the viscous coefficient
-// nu dt |k|^2, which is formed in FP64 and rounded once.  |k|^2 and the
-// wavenumbers are integers below 2^24, exact in FP32; dt and the RK
-// coefficients are rounded once per launch (rk = (dt, a, b) as floats).
-template <int ST>
-__device__ __forceinline__ void update_point_f32(const UpdIn<float> &in, UpdOut<float> &out,
-                                                 const Geo &g, float dtf, double nudt, float ra,
-                                                 float rb, int i, int j, int col) {
-  const int ikx = kwave(i, g.n), iky = kwave(j, g.n);
-  const float kx = (float)ikx, ky = (float)iky, kz = (float)col;
-  const bool inm = (ikx < 0 ? -ikx : ikx) <= g.kcut && (iky < 0 ? -iky : iky) <= g.kcut &&
-                   col <= g.kcut;
-  const float2 zero = make_float2(0.f, 0.f);
-  float2 du = inm ? cscale(in.n[0], dtf) : zero;
-  float2 dv = inm ? cscale(in.n[1], dtf) : zero;
-  float2 dw = inm ? cscale(in.n[2], dtf) : zero;
-  const int ikk = ikx * ikx + iky * iky + col * col;
-  const float kk = (float)ikk;
-  float2 P;
-  if (ikk > 0) {
-    P.x = __fdiv_rn(du.x * kx + dv.x * ky + dw.x * kz, kk);
-    P.y = __fdiv_rn(du.y * kx + dv.y * ky + dw.y * kz, kk);
-  } else {
-    P = zero;
-  }
-  const float c = (float)(nudt * (double)ikk);
-  du = make_float2(du.x - (P.x * kx + c * in.us[0].x), du.y - (P.y * kx + c * in.us[0].y));
-  dv = make_float2(dv.x - (P.x * ky + c * in.us[1].x), dv.y - (P.y * ky + c * in.us[1].y));
-  dw = make_float2(dw.x - (P.x * kz + c * in.us[2].x), dw.y - (P.y * kz + c * in.us[2].y));
-  out.p = P;
-  auto axpy = [](float2 x, float s, float2 y) { return make_float2(x.x + s * y.x, x.y + s * y.y); };
-  const float2 d[3] = {du, dv, dw};
-#pragma unroll
-  for (int f = 0; f < 3; f++) {
-    if (ST == 0) {  // us == u0
-      out.o1[f] = axpy(in.us[f], rb, d[f]);
-      out.o2[f] = axpy(in.us[f], ra, d[f]);
-    } else if (ST < 3) {
-      out.o1[f] = axpy(in.z[f], rb, d[f]);
-      out.o2[f] = axpy(in.a[f], ra, d[f]);
-    } else {
-      out.o1[f] = axpy(in.a[f], ra, d[f]);
-    }
-  }
-}
-
-constexpr int UPD_THREADS = 128;
-// adjacent points per vector access: two float2 make one 16-byte access
-template <class R>
-struct UpdVec;
-template <>
-struct UpdVec<double> {
-  static constexpr int VP = 1;
-  using T = double2;
-  __device__ static double2 get(const T &v, int) { return v; }
-  __device__ static T pack(const double2 *c) { return c[0]; }
-};
-template <>
-struct UpdVec<float> {
-  static constexpr int VP = 2;
-  using T = float4;
-  __device__ static float2 get(const T &v, int k) {
-    return k ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
-  }
-  __device__ static T pack(const float2 *c) { return make_float4(c[0].x, c[0].y, c[1].x, c[1].y); }
-};
-
-// grid: (ceil(n^2 nfp / VP / UPD_THREADS), nruns).  Thread = VP adjacent
-// points of the padded slot (padding columns included and skipped), so that
-// the row, kx and ky of a point come from divisions by compile-time constants.
-// One chunk of UPD_THREADS threads: chunk b.x of run b.y.
-template <class R, int N, int ST>
-__device__ __forceinline__ void update_body(const cx<R> *__restrict__ nl, const Geo &g,
-                                            const StageArgs<R> &sa, const Blk b) {
-  using VT = UpdVec<R>;
-  using V = typename VT::T;
-  constexpr int VP = VT::VP;
-  constexpr int NF = N / 2 + 1;
-  constexpr int NFP = (NF + PitchW<R>::W - 1) / PitchW<R>::W * PitchW<R>::W;
-  constexpr unsigned NPAD = (unsigned)N * N * NFP;
-  static_assert(NFP % VP == 0, "vector access must not straddle rows");
-  const unsigned q0 = ((unsigned)b.x * (unsigned)UPD_THREADS + (unsigned)b.tid) * VP;
-  if (q0 >= NPAD) return;
-  const unsigned row = q0 / NFP;
-  const int col0 = (int)(q0 - row * NFP);
-  if (col0 >= NF) return;
-  const long long rb = (long long)b.y * g.run_spec;
-  const double nu = sa.coef[2 * b.y], dt = sa.coef[2 * b.y + 1];
-  const long long vo = (rb + q0) / VP, vs = g.slot / VP;  // vector index, slot stride
-  const V *vn = (const V *)nl, *vus = (const V *)sa.us, *vz = (const V *)sa.u0,
-          *va = (const V *)sa.acc;
-  V ln[3], lus[3], lz[3], la[3];
-  // N is read only where some point of the access lies inside the 2/3 rule
-  const int ikx = kwave((int)(row / N), N), iky = kwave((int)(row % N), N);
-  const bool need_n = (ikx < 0 ? -ikx : ikx) <= g.kcut && (iky < 0 ? -iky : iky) <= g.kcut &&
-                      col0 <= g.kcut;
-#pragma unroll
-  for (int f = 0; f < 3; f++) {
-    ln[f] = need_n ? vn[f * vs + vo] : V{};
-    lus[f] = vus[f * vs + vo];
-    if (ST == 1 || ST == 2) lz[f] = vz[f * vs + vo];
-    if (ST != 0) la[f] = va[f * vs + vo];
-  }
-  UpdOut<R> res[VP];
-#pragma unroll
-  for (int v = 0; v < VP; v++) {
-    if (col0 + v < NF) {
-      UpdIn<R> in;
+  } else if constexpr (ST >= 0) {
+    // packed stage inputs, this thread's column of field 0 of stage 1
+    const unsigned crs = (unsigned)g.mk * g.mp;
+    C *rk = a.rk + rb + (unsigned)(iky < 0 ? iky + g.mk : iky) * g.mp + col;
+    auto crow = [&](int ik) -> long long {
+      return (long long)((unsigned)(ik < 0 ? ik + g.mk : ik) * crs);
+    };
+    // state and stage inputs of a point, loaded a point ahead (as far as the
+    // compiler knows a store may alias a later load) except in stage 3, whose
+    // four triples leave no registers for it
+    constexpr bool AHEAD = ST < 3;
+    struct In {
+      C z[3], us[3], r1[3], r2[3];
+    };
+    auto load = [&](In &q, int e) {
+      const int ik = kwave(t + T * e, N);
+      const bool in = zin && kin(ik);
 #pragma unroll
       for (int f = 0; f < 3; f++) {
-        in.n[f] = VT::get(ln[f], v);
-        in.us[f] = VT::get(lus[f], v);
-        if (ST == 1 || ST == 2) in.z[f] = VT::get(lz[f], v);
-        if (ST != 0) in.a[f] = VT::get(la[f], v);
+        q.z[f] = ok ? ldcg(u0 + at(e) + f * g.slot) : czero<C>();
+        if constexpr (ST > 0)
+          q.us[f] = in ? ldcg(rk + crow(ik) + (3 * (ST - 1) + f) * g.slotc) : czero<C>();
+        if constexpr (ST == 3) {
+          q.r1[f] = in ? ldcg(rk + crow(ik) + f * g.slotc) : czero<C>();
+          q.r2[f] = in ? ldcg(rk + crow(ik) + (3 + f) * g.slotc) : czero<C>();
+        }
       }
-      if constexpr (sizeof(R) == 4)
-        update_point_f32<ST>(in, res[v], g, (float)dt, nu * dt, (float)sa.a, (float)sa.b,
-                             (int)(row / N), (int)(row % N), col0 + v);
-      else
-        update_point<R, ST>(in, res[v], g, sa, nu, dt, (int)(row / N), (int)(row % N), col0 + v);
+    };
+    line_fft<N, P, true>(v, t, st, xb, idx, sync);
+    copies_done();
+#pragma unroll
+    for (int e = 0; e < E; e++) {  // N_x takes N_y's place
+      const C y = landed(s0, e);
+      s0[e * TH] = v[e];
+      v[e] = y;
+    }
+    line_fft<N, P, true>(v, t, st, xb, idx, sync);
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const C y = landed(s1, e);
+      s1[e * TH] = v[e];
+      v[e] = y;
+    }
+    In in0, in1;
+    if (AHEAD) load(in0, 0);
+    line_fft<N, P, true>(v, t, st, xb, idx, sync);
+    const R dtr = (R)dt, ky = (R)iky, kz = (R)col;
+    auto update = [&](const In &q, int e) {
+      const int ik = kwave(t + T * e, N);
+      const int ikk = ik * ik + kyz;
+      const R c = (R)(nudt * (double)ikk);  // formed in FP64, rounded once
+      C r[3];
+      if (zin && kin(ik)) {
+        const R kk = (R)ikk, k[3] = {(R)ik, ky, kz};
+        C n[3] = {s0[e * TH], s1[e * TH], v[e]};
+#pragma unroll
+        for (int f = 0; f < 3; f++) n[f] = cmk<C>(mul_rn(n[f].x, dtr), mul_rn(n[f].y, dtr));
+        auto dot = [&](R x, R y, R z) -> R {
+          return fma_rn(z, k[2], fma_rn(y, k[1], mul_rn(x, k[0])));
+        };
+        C pr = czero<C>();
+        if (ikk > 0) {
+          pr.x = div_rn(dot(n[0].x, n[1].x, n[2].x), kk);
+          pr.y = div_rn(dot(n[0].y, n[1].y, n[2].y), kk);
+        }
+#pragma unroll
+        for (int f = 0; f < 3; f++) {
+          const C us = ST == 0 ? q.z[f] : q.us[f];
+          const C dd = cmk<C>(n[f].x - fma_rn(pr.x, k[f], mul_rn(c, us.x)),
+                              n[f].y - fma_rn(pr.y, k[f], mul_rn(c, us.y)));
+          if constexpr (ST < 3) {
+            constexpr R bs = ST < 2 ? R(0.5) : R(1);
+            r[f] = cmk<C>(fma_rn(bs, dd.x, q.z[f].x), fma_rn(bs, dd.y, q.z[f].y));
+            rk[crow(ik) + (3 * ST + f) * g.slotc] = r[f];
+          } else {
+            auto sum = [](R q0, R q1, R q2, R q3, R du) -> R {
+              const R inc = (q1 - q0) + R(2) * (q2 - q0) - R(2) * (q3 - q0);
+              return fma_rn(inc, R(1.0 / 3.0), fma_rn(du, R(1.0 / 6.0), q3));
+            };
+            r[f] = cmk<C>(sum(q.z[f].x, q.r1[f].x, q.r2[f].x, us.x, dd.x),
+                          sum(q.z[f].y, q.r1[f].y, q.r2[f].y, us.y, dd.y));
+          }
+        }
+        if (ST == 3 && a.ph) a.ph[rb + base + at(e)] = pr;
+      } else {
+        const R m = lin_coef<ST>(c);
+#pragma unroll
+        for (int f = 0; f < 3; f++)
+          r[f] = cmk<C>(fma_rn(m, q.z[f].x, q.z[f].x), fma_rn(m, q.z[f].y, q.z[f].y));
+      }
+      if (ST == 3 && ok) {
+#pragma unroll
+        for (int f = 0; f < 3; f++) u0[at(e) + f * g.slot] = r[f];
+      }
+      v[e] = r[0];
+      s0[e * TH] = r[1];
+      s1[e * TH] = r[2];
+    };
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      In &cur = AHEAD && e % 2 ? in1 : in0, &nxt = AHEAD && e % 2 ? in0 : in1;
+      if (!AHEAD) load(cur, e);
+      if (AHEAD && e + 1 < E) load(nxt, e + 1);
+      update(cur, e);
     }
   }
-  V *o1 = (V *)(ST == 3 ? sa.u0 : sa.next), *o2 = (V *)sa.acc, *vp = (V *)sa.ph;
-  if (col0 + VP - 1 < NF) {
-    cx<R> t1[VP], t2[VP], tp[VP];
+  if constexpr (!TAIL) return;
+
+  // x backward of u, and of i kx f and f for f = v, w
+  auto back = [&](int slot) {  // transform v into a work slot
+    line_fft<N, P, false>(v, t, st, xb, idx, sync);
+    if (ok) {
+      C *dst = wk + slot * g.slot;
 #pragma unroll
-    for (int f = 0; f < 3; f++) {
-#pragma unroll
-      for (int v = 0; v < VP; v++) {
-        t1[v] = res[v].o1[f];
-        t2[v] = res[v].o2[f];
-      }
-      o1[f * vs + vo] = VT::pack(t1);
-      if (ST != 3) o2[f * vs + vo] = VT::pack(t2);
+      for (int e = 0; e < E; e++) dst[at(e)] = v[e];
     }
-    if (vp) {
+  };
+  back(SU);
 #pragma unroll
-      for (int v = 0; v < VP; v++) tp[v] = res[v].p;
-      vp[vo] = VT::pack(tp);
-    }
-  } else {  // the row's last valid column: store its point alone
-    const long long o = rb + q0;
-    cx<R> *s1 = ST == 3 ? sa.u0 : sa.next;
+  for (int f = 1; f < 3; f++) {
+    const C *s = f == 1 ? s0 : s1;
 #pragma unroll
-    for (int f = 0; f < 3; f++) {
-      s1[f * g.slot + o] = res[0].o1[f];
-      if (ST != 3) sa.acc[f * g.slot + o] = res[0].o2[f];
+    for (int e = 0; e < E; e++) {
+      const R k = (R)kwave(t + T * e, N);
+      const C z = s[e * TH];
+      v[e] = cmk<C>(mul_rn(-k, z.y), mul_rn(k, z.x));  // i kx f
     }
-    if (sa.ph) sa.ph[o] = res[0].p;
+    back(f == 1 ? SOMZ : SDWDX);
+#pragma unroll
+    for (int e = 0; e < E; e++) v[e] = s[e * TH];
+    back(f == 1 ? SV : SW);
   }
 }
 
-template <class R, int N, int ST>
-__global__ void __launch_bounds__(UPD_THREADS)
-    k_update(const cx<R> *__restrict__ nl, Geo g, StageArgs<R> sa) {
-  update_body<R, N, ST>(nl, g, sa, launch_blk());
+// grid: (ceil(nf / W), n, nruns); block: XC::THREADS
+template <class R, int N, int ST, bool TAIL>
+__global__ void __launch_bounds__(XC<R, N>::THREADS, XC<R, N>::MINB)
+    k_xstage(XArgs<R> a, const cx<R> *__restrict__ twg, Geo g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  xstage_body<R, N, ST, TAIL>(a, twg, g, launch_blk(), BlockSync{}, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

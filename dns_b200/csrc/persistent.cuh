@@ -1,13 +1,14 @@
 // persistent.cuh -- one cooperative kernel launch per RK4 step of a whole
 // ensemble (dns_ens in its persistent schedule).
 //
-// The batched schedule steps an ensemble with 24 launches per size group
-// (four RK stages of six passes), size groups as concurrent branches of a
+// The batched schedule steps an ensemble with 16 launches per size group
+// (four RK stages of four kernels), size groups as concurrent branches of a
 // CUDA graph.  Here a single cooperative launch, of as many blocks as fit
-// on the GPU at once, walks the same 24 phases for every run of every size:
-// in each phase the work items of all groups (the blocks the standalone
-// kernels would launch: column tiles, z line groups, update chunks) are
-// pooled and dealt out to the blocks, which run the same pass bodies as the
+// on the GPU at once, walks a step's phases (the x transform of the state,
+// then the four kernels of each stage) for every run of every size: in each
+// phase the work items of all groups (the blocks the standalone kernels
+// would launch: column tiles, z line groups, x tiles) are pooled and dealt
+// out to the blocks, which run the same pass bodies as the
 // standalone kernels (kernels.cuh), so each run's state is bit-identical to
 // the batched schedule's.  Phases are separated by a grid-wide barrier.
 //
@@ -26,9 +27,9 @@ namespace dnsb {
 
 constexpr int PBS = 128;        // threads per block
 constexpr int PMAXG = 4;        // size groups
-constexpr int PPHASES = 24;     // 4 RK stages x 6 passes
+constexpr int PPHASES = 17;     // the x transform of the state, 4 RK stages x 4 kernels
 enum : unsigned { PERR_BARRIER_TIMEOUT = 1u };
-enum { PK_COL = 0, PK_Z = 1, PK_UPD = 2 };
+enum { PK_COL = 0, PK_Z = 1, PK_X = 2 };
 
 // register cap: FP64's z pass needs 255 registers (2 blocks of 128
 // threads), FP32's 170 (3 blocks)
@@ -40,13 +41,13 @@ struct PMinB {
 template <class R>
 struct PPhase {
   int kind;          // PK_*
-  int axis, fwd;     // column pass
-  int sub;           // z-pass KIND or update stage
+  int fwd;           // y column pass: direction
+  int sub;           // z-pass KIND or x-pass stage
   int gx, gy, gz;    // work items: the grid of the standalone launch
   int tpi;           // threads per item
   int smem;          // shared bytes per item
   ColJobs jobs;
-  StageArgs<R> sa;
+  XArgs<R> xa;
 };
 
 template <class R>
@@ -129,17 +130,10 @@ template <class R, int N, class Sync>
 __device__ __forceinline__ void p_item_n(const PGroup<R> &G, const PPhase<R> &P, const Blk b,
                                          Sync sync, unsigned char *sm) {
   if (P.kind == PK_COL) {
-    if (P.axis == 0) {
-      if (P.fwd)
-        colpass_body<R, N, 0, true>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
-      else
-        colpass_body<R, N, 0, false>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
-    } else {
-      if (P.fwd)
-        colpass_body<R, N, 1, true>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
-      else
-        colpass_body<R, N, 1, false>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
-    }
+    if (P.fwd)
+      colpass_body<R, N, 1, true>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
+    else
+      colpass_body<R, N, 1, false>(G.S, G.S, G.tw, G.g, P.jobs, b, sync, sm);
   } else if (P.kind == PK_Z) {
     if (P.sub == 0)
       zstage_body<R, N, 0>(G.work, G.stale, G.tw, G.g, G.invn3, b, sync, sm);
@@ -148,14 +142,16 @@ __device__ __forceinline__ void p_item_n(const PGroup<R> &G, const PPhase<R> &P,
     else
       zstage_body<R, N, 2>(G.work, G.stale, G.tw, G.g, G.invn3, b, sync, sm);
   } else {
-    if (P.sub == 0)
-      update_body<R, N, 0>(G.work, G.g, P.sa, b);
+    if (P.sub < 0)
+      xstage_body<R, N, -1, true>(P.xa, G.tw, G.g, b, sync, sm);
+    else if (P.sub == 0)
+      xstage_body<R, N, 0, true>(P.xa, G.tw, G.g, b, sync, sm);
     else if (P.sub == 1)
-      update_body<R, N, 1>(G.work, G.g, P.sa, b);
+      xstage_body<R, N, 1, true>(P.xa, G.tw, G.g, b, sync, sm);
     else if (P.sub == 2)
-      update_body<R, N, 2>(G.work, G.g, P.sa, b);
+      xstage_body<R, N, 2, true>(P.xa, G.tw, G.g, b, sync, sm);
     else
-      update_body<R, N, 3>(G.work, G.g, P.sa, b);
+      xstage_body<R, N, 3, false>(P.xa, G.tw, G.g, b, sync, sm);
   }
 }
 
@@ -190,7 +186,7 @@ __global__ void __launch_bounds__(PBS, PMinB<R>::value)
       const int per = PBS / P.tpi;
       const int sub = (int)threadIdx.x / P.tpi;
       const int item = v * per + sub;
-      if (item < P.gx * P.gy * P.gz) {
+      if (sub < per && item < P.gx * P.gy * P.gz) {
         const Blk b{item % P.gx, (item / P.gx) % P.gy, item / (P.gx * P.gy),
                     (int)threadIdx.x % P.tpi, P.tpi};
         // every item synchronises on its own barrier (one body per pass)

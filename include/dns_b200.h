@@ -137,7 +137,8 @@ typedef struct {
   unsigned flags;
   size_t device_bytes;     /* device memory held by the context */
   size_t slot_bytes;       /* bytes of one padded spectral field */
-  int kernels_per_step;    /* kernel launches in one RK4 step */
+  int kernels_per_step;    /* passes of one RK4 step, the entries that
+                              dns_time_kernels writes */
 } dns_info_t;
 int dns_get_info(dns_ctx *ctx, dns_info_t *info);
 /* The kernel schedule the library's autotuner chose for this context's grid
@@ -161,10 +162,12 @@ void *dns_get_stream(dns_ctx *ctx);
 /* Wait for all work queued on the context's stream. */
 int dns_synchronize(dns_ctx *ctx);
 
-/* Time each kernel of the step: runs nsteps steps launch by launch with CUDA
+/* Time each pass of the step: runs nsteps steps launch by launch with CUDA
  * events between kernels and writes the mean time in milliseconds of each of
- * the kernels_per_step launches of a step into ms[] (stage-major order:
- * stage 0 passes A..E, stage 1 ..., stage 3).  The state advances by
+ * the kernels_per_step passes of a step into ms[] (stage-major order: stage 0
+ * passes A x-inverse, B y-inverse, C z, D y-forward, E1 x-forward, E2 update,
+ * stage 1 ..., stage 3).  A stage's E1 and E2 and the next stage's A are one
+ * kernel, whose time is divided equally among them.  The state advances by
  * nsteps. */
 int dns_time_kernels(dns_ctx *ctx, double nu, double dt, long nsteps, double *ms);
 
@@ -173,13 +176,13 @@ int dns_time_kernels(dns_ctx *ctx, double nu, double dt, long nsteps, double *ms
  * process-level ensembles (run.sh / hal.sh run one dns per core).  Runs of
  * any grid sizes and viscosities advance together, each following main.c's
  * step exactly (stale velocity included), under one of two schedules:
- *   batched     runs of equal n share batched kernel launches (24 per step),
+ *   batched     runs of equal n share batched kernel launches (16 per step),
  *               groups of different n run as concurrent branches of one
  *               CUDA graph launch per step;
  *   persistent  one cooperative kernel launch per step (captured in a CUDA
- *               graph) walks the 24 passes of every run of every size, the
- *               passes separated by grid-wide barriers (grid sizes 32, 64
- *               and 128, at most four distinct sizes).
+ *               graph) walks the passes of every run of every size, the
+ *               passes separated by grid-wide barriers (grid sizes 64 and
+ *               128, at most four distinct sizes).
  * Both give bit-identical states.  dns_ens_create times both on the fresh
  * ensemble and keeps the faster (its autotuner) unless a flag forces one:
  * DNS_FLAG_ENS_BATCHED or DNS_FLAG_ENS_PERSISTENT (DNS_ERR_UNSUPPORTED when
@@ -227,8 +230,8 @@ int dns_ens_synchronize(dns_ens *e);
  * recomputed from `snapshots` stored step states (>= 1, the initial state
  * included) placed by a binomial split of the step range, so memory is
  * independent of nsteps: the snapshots (3 spectral and 3 real fields each)
- * plus a fixed work set (41 spectral and 45 real fields, the step's own
- * state included; 256^3 FP64 with 20 snapshots: about 28 GB).  Any output pointer may be NULL;
+ * plus a fixed work set (30 spectral and 45 real fields, the step's own
+ * state included; 256^3 FP64 with 20 snapshots: about 27 GB).  Any output pointer may be NULL;
  * with all four gradient pointers NULL only the forward sweep runs (J
  * alone). */
 int dns_adjoint_energy(long n, const double *U, const double *V, const double *W, double nu,
