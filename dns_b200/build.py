@@ -22,7 +22,9 @@ INCLUDE = os.path.join(ROOT, "include")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-O3", "-lineinfo", "-std=c++17", "-split-compile=0",
+    "-O3", "-lineinfo", "-std=c++17",
+    # kernels are compiled in one translation unit and launched from another
+    "-static-global-template-stub=false", "-diag-suppress", "20279,20281",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
 ]
 

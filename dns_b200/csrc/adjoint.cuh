@@ -81,29 +81,6 @@ struct StageIn {
   }
 };
 
-// out = U_s on 3 slots
-template <class C>
-__global__ void k_stage_input(StageIn<C> us, C *__restrict__ out, Geo g) {
-  DNSB_FOR_POINTS(g) {
-    const PointK p = point_k(g, q);
-#pragma unroll
-    for (int f = 0; f < 3; f++) out[f * g.slot + p.o] = us.at(g, p, f);
-  }
-}
-
-// out = curl(in) on 3 slots
-template <class C>
-__global__ void k_curl(const C *__restrict__ in, C *__restrict__ out, Geo g) {
-  DNSB_FOR_POINTS(g) {
-    const PointK p = point_k(g, q);
-    cd ox, oy, oz;
-    curl_at(p, to_d(in[p.o]), to_d(in[g.slot + p.o]), to_d(in[2 * g.slot + p.o]), ox, oy, oz);
-    out[p.o] = from_d<C>(ox);
-    out[g.slot + p.o] = from_d<C>(oy);
-    out[2 * g.slot + p.o] = from_d<C>(oz);
-  }
-}
-
 // out = (m dt Pi(ldU)) / w_z : the adjoint of N_hat, divided by the c2r
 // weights so that a plain c2r of `out` is r2c^T of m dt Pi(ldU)
 template <class C>

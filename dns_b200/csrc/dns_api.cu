@@ -18,8 +18,8 @@
 #include "dns_b200.h"
 #include "adjoint.cuh"
 #include "init.cuh"
-#include "kernels.cuh"
-#include "persistent.cuh"
+#include "ops.cuh"
+#include "instances.cuh"
 
 #include <math.h>
 #include <stdio.h>
@@ -38,14 +38,6 @@ using namespace dnsb;
 namespace {
 
 thread_local std::string g_last_error;
-
-enum { SLOT_SA = 0, SLOT_RK = 3, SLOT_WORK = 7, SLOT_P = 14, NSLOTS = 15 };
-// passes of an RK stage, as dns_time_kernels reports them: A x-inverse, B
-// y-inverse, C z fused, D y-forward, E1 x-forward, E2 pointwise update
-enum { PASSES_PER_STAGE = 6 };
-// the launches that run them: B, C, D and X, which is a stage's E1 and E2 and
-// the next stage's A in one kernel
-enum { K_B = 0, K_C = 1, K_D = 2, K_X = 3, KERNELS_PER_STAGE = 4 };
 
 int fail(int code, const char *what, const char *file, int line) {
   char buf[512];
@@ -116,51 +108,6 @@ namespace dnsb {
 void set_last_error(const char *msg) { g_last_error = msg; }
 }  // namespace dnsb
 
-// A group: nruns runs of one grid size and precision in one arena, stepped
-// by the same (batched) kernel launches.  A dns_ctx is a group of one run;
-// a dns_ens holds one group per distinct grid size.
-struct Group {
-  long n = 0;
-  int precision = 0;
-  unsigned flags = 0;
-  int nruns = 1;
-  size_t csize = 16;      // bytes of one complex element
-  size_t rsize = 8;       // bytes of one real element
-  Geo g{};
-  char *arena = nullptr;
-  size_t arena_bytes = 0;
-  void *S = nullptr;      // spectral slots [nruns][NSLOTS][slot]
-  void *stale = nullptr;  // stale real velocity [nruns][3][n^3]
-  void *tw = nullptr;     // twiddles exp(-2 pi i k / n)
-  double4 *diag_part = nullptr;  // [nruns][diag_blocks]
-  double4 *diag_out = nullptr;   // [nruns]
-  double *coef = nullptr;        // [nruns][2]: nu, dt
-  int diag_blocks = 0;
-  double *realbuf = nullptr;     // [4][n^3] float64, allocated on first field read
-  // column-pass register schedules [axis][forward] picked by the autotuner
-  // for this group's launches, and the run count they were timed on
-  int pick[2][2] = {{0, 0}, {0, 0}};
-  int tune_runs = 1;
-
-  char *slot_ptr(int run, int s) const {
-    return (char *)S + ((size_t)run * g.run_spec + (size_t)s * g.slot) * csize;
-  }
-  // float64 staging for host transfers of the FP32 path: the run's work
-  // slots (7 * n^2 * nfp * 8 bytes >= 3 n^3 * 8 and >= 3 n^2 nf * 16)
-  double *staging(int run) const { return (double *)slot_ptr(run, SLOT_WORK); }
-  // the same arena seen as a batch of one run
-  Group one(int run) const {
-    Group v = *this;
-    v.nruns = 1;
-    v.S = slot_ptr(run, 0);
-    v.stale = (char *)stale + (size_t)run * g.run_real * rsize;
-    v.diag_part = diag_part + (size_t)run * diag_blocks;
-    v.diag_out = diag_out + run;
-    v.coef = coef + 2 * run;
-    return v;
-  }
-};
-
 struct dns_ctx {
   Group grp;
   cudaStream_t stream = nullptr;
@@ -201,475 +148,6 @@ namespace {
 // main.c:15-16 (the forward step has them written out in xstage_body)
 constexpr double RK_A[4] = {1 / 6.0, 1 / 3.0, 1 / 3.0, 1 / 6.0};
 constexpr double RK_B[3] = {0.5, 0.5, 1.0};
-
-ColJobs jobs_empty(int njobs) {
-  ColJobs j;
-  for (int q = 0; q < 8; q++)
-    j.in_slot[q] = 0, j.out_slot[q] = -1, j.der_slot[q] = -1, j.add_slot[q] = -1;
-  j.njobs = njobs;
-  j.masked = 0;
-  return j;
-}
-ColJobs jobs_pass_b(bool first) {
-  ColJobs j = jobs_empty(4);
-  const int w = SLOT_WORK;
-  // u, and omega_z = dv/dx - i ky u over the dv/dx slot (same tile, same block)
-  j.in_slot[0] = w + SU; j.out_slot[0] = w + SU; j.der_slot[0] = w + SOMZ; j.add_slot[0] = w + SOMZ;
-  j.in_slot[1] = w + SV; j.out_slot[1] = w + SV;
-  // the first stage reads the stale real velocity, so W itself is not needed
-  j.in_slot[2] = w + SW; j.out_slot[2] = first ? -1 : w + SW; j.der_slot[2] = w + SDWDY;
-  j.in_slot[3] = w + SDWDX; j.out_slot[3] = w + SDWDX;
-  return j;
-}
-ColJobs jobs_map(const int *in, const int *out, int cnt) {
-  ColJobs j = jobs_empty(cnt);
-  for (int q = 0; q < cnt; q++) j.in_slot[q] = in[q], j.out_slot[q] = out[q];
-  return j;
-}
-
-template <class R, int N>
-struct Ops {
-  using Real = R;
-  using C = cx<R>;
-  static constexpr int Nval = N;
-  static constexpr int E = Plan<N>::E;
-  template <int AXIS>
-  static constexpr int CW = ColW<R, AXIS, N>::W;
-  template <int AXIS>
-  static constexpr int CT = (N / E) * CW<AXIS>;
-  template <int AXIS>
-  static constexpr size_t COL_SMEM = (size_t)(N + N * CW<AXIS>) * sizeof(C);
-  static constexpr size_t Z_SMEM = (size_t)(2 * N + ZCfg<N>::LINES * ZCfg<N>::XB) * sizeof(C);
-  template <int KIND>
-  static constexpr size_t ZS_SMEM = ZC<R, N, KIND>::SMEM;
-  using X = XC<R, N>;
-  static constexpr size_t XS_SMEM = X::SMEM;
-  // the z pass can keep its real velocity and vorticity (k_zstage_keep)
-  static constexpr bool ZKEEP = ZC<R, N, 1>::S2 || ZC<R, N, 1>::F32;
-
-  // Column-pass register schedules.  Candidate I of a pass is the same
-  // kernel compiled with a minimum of ColCands::m[I] resident blocks per SM
-  // (0: the compiler's own register choice); the candidates differ only in
-  // register allocation, so every one computes bit-identical results.  The
-  // autotuner (tune()) times them once per process, size and batch shape
-  // (the run count it times on) and keeps the fastest; sizes below 64 have
-  // the compiler's choice only.
-  using ColFn = void (*)(const C *, C *, const C *, Geo, ColJobs);
-  template <int AXIS>
-  using Cands = ColCands<(N >= 64 ? (N / Plan<N>::E) * ColW<R, AXIS, N>::W : 0), (int)sizeof(C)>;
-  template <int AXIS, bool FWD, int I>
-  static ColFn col_cand() {
-    constexpr int m = Cands<AXIS>::m[I];
-    if constexpr (m == 0)
-      return k_colpass<R, N, AXIS, FWD>;
-    else
-      return k_colpass_minb<R, N, AXIS, FWD, m>;
-  }
-  template <int AXIS, bool FWD, int I = 0>
-  static ColFn col_cand_at(int i) {
-    if constexpr (I + 1 < Cands<AXIS>::n) {
-      if (i != I) return col_cand_at<AXIS, FWD, I + 1>(i);
-    }
-    return col_cand<AXIS, FWD, I>();
-  }
-  // chosen candidate of [AXIS][FWD] and the measured time per launch (ms)
-  // of every candidate, per tuning run count
-  struct TuneRec {
-    int pick[2][2];
-    float ms[2][2][16];
-  };
-  static inline std::map<int, TuneRec> tune_cache;
-  static inline std::mutex tune_mu;  // guards tune_cache
-  template <int AXIS, bool FWD>
-  static ColFn colkern(const Group &G) {
-    return col_cand_at<AXIS, FWD>(G.pick[AXIS][FWD]);
-  }
-  // runs a batch is tuned on: all of them up to the volume of two 256^3
-  // runs, which fills the GPU like any larger batch
-  static int tune_runs(int nruns) {
-    long long cap = 2LL * 256 * 256 * 256 / ((long long)N * N * N);
-    if (cap < 1) cap = 1;
-    return (int)(nruns < cap ? nruns : cap);
-  }
-
-  template <class K>
-  static cudaError_t allow(K kern, size_t smem) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  template <int AXIS, bool FWD>
-  static cudaError_t allow_cands() {
-    cudaError_t e = cudaSuccess;
-    for (int i = 0; i < Cands<AXIS>::n && e == cudaSuccess; i++)
-      e = allow(col_cand_at<AXIS, FWD>(i), COL_SMEM<AXIS>);
-    return e;
-  }
-  static cudaError_t setup() {
-    cudaError_t e;
-    if ((e = allow_cands<0, false>())) return e;
-    if ((e = allow_cands<0, true>())) return e;
-    if ((e = allow_cands<1, false>())) return e;
-    if ((e = allow_cands<1, true>())) return e;
-    if ((e = allow(k_zstage<R, N, 0>, ZS_SMEM<0>))) return e;
-    if ((e = allow(k_zstage<R, N, 1>, ZS_SMEM<1>))) return e;
-    if ((e = allow(k_zstage<R, N, 2>, ZS_SMEM<2>))) return e;
-    if constexpr (ZKEEP) {
-      if ((e = allow(k_zstage_keep<R, N, 0>, ZS_SMEM<0>))) return e;
-      if ((e = allow(k_zstage_keep<R, N, 1>, ZS_SMEM<1>))) return e;
-    }
-    if ((e = allow(k_xstage<R, N, -1, true>, XS_SMEM))) return e;
-    if ((e = allow(k_xstage<R, N, 0, true>, XS_SMEM))) return e;
-    if ((e = allow(k_xstage<R, N, 1, true>, XS_SMEM))) return e;
-    if ((e = allow(k_xstage<R, N, 2, true>, XS_SMEM))) return e;
-    if ((e = allow(k_xstage<R, N, 3, true>, XS_SMEM))) return e;
-    if ((e = allow(k_xstage<R, N, 3, false>, XS_SMEM))) return e;
-    if ((e = allow(k_zr2c<R, N>, Z_SMEM))) return e;
-    if ((e = allow(k_zc2r<R, N>, Z_SMEM))) return e;
-    return cudaSuccess;
-  }
-
-  // ---- autotuner of the column-pass register schedules ----
-  template <int AXIS, bool FWD>
-  static cudaError_t time_cands(Group &Gt, cudaStream_t st, const ColJobs &jobs, cudaEvent_t e0,
-                                cudaEvent_t e1, int force, int force_m, TuneRec &rec) {
-    constexpr int n = Cands<AXIS>::n;
-    int &pick = Gt.pick[AXIS][FWD];
-    if (force_m >= 0) {  // a given register schedule: its candidate, else the compiler's
-      pick = 0;
-      for (int i = 0; i < n; i++)
-        if (Cands<AXIS>::m[i] == force_m) pick = i;
-      rec.pick[AXIS][FWD] = pick;
-      return cudaSuccess;
-    }
-    int best = 0;
-    for (int i = 0; i < n; i++) {
-      pick = i;
-      colpass_io<AXIS, FWD>(Gt, st, (C *)Gt.S, (C *)Gt.S, jobs, Gt.nruns);  // warm-up
-      cudaError_t e = cudaEventRecord(e0, st);
-      for (int r = 0; r < 3 && e == cudaSuccess; r++) {
-        colpass_io<AXIS, FWD>(Gt, st, (C *)Gt.S, (C *)Gt.S, jobs, Gt.nruns);
-        e = cudaGetLastError();
-      }
-      if (e == cudaSuccess) e = cudaEventRecord(e1, st);
-      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-      float ms = 0.f;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      if (e != cudaSuccess) return e;
-      rec.ms[AXIS][FWD][i] = ms / 3.f;
-      if (rec.ms[AXIS][FWD][i] < rec.ms[AXIS][FWD][best]) best = i;
-    }
-    pick = force >= 0 ? (force < n ? force : n - 1) : best;
-    rec.pick[AXIS][FWD] = pick;
-    return cudaSuccess;
-  }
-  // Time every register schedule of the four column passes (y: the job
-  // tables of an RK stage, x: three fields, as the initial transform and the
-  // field reads run them; batched over the group's first tune_runs(nruns)
-  // runs, on their work slots, whose contents do not matter to an FFT's
-  // timing) and keep the fastest of each; once per process, size and tuning
-  // run count.  The group launches with the picks (G.pick).  DNS_B200_TUNE=0 keeps the compiler's schedule,
-  // DNS_B200_TUNE=f<k> forces candidate k (the last where there are fewer),
-  // DNS_B200_TUNE=m<a>,<b>,<c>,<d> the schedules of min blocks/SM a, b, c, d
-  // for the x inverse, x forward, y inverse and y forward passes (as
-  // dns_get_schedule reports them; a value that is not a candidate means
-  // the compiler's).
-  static cudaError_t tune(Group &G, cudaStream_t st, bool *ran) {
-    std::lock_guard<std::mutex> lock(tune_mu);
-    *ran = false;
-    G.tune_runs = tune_runs(G.nruns);
-    auto it = tune_cache.find(G.tune_runs);
-    if (it != tune_cache.end()) {
-      memcpy(G.pick, it->second.pick, sizeof G.pick);
-      return cudaSuccess;
-    }
-    TuneRec rec{};
-    const char *env = getenv("DNS_B200_TUNE");
-    if (env && strcmp(env, "0") == 0) {
-      tune_cache[G.tune_runs] = rec;
-      memset(G.pick, 0, sizeof G.pick);
-      return cudaSuccess;
-    }
-    const int force = (env && env[0] == 'f') ? atoi(env + 1) : -1;
-    int fm[4] = {-1, -1, -1, -1};  // x inverse, x forward, y inverse, y forward
-    if (env && env[0] == 'm') {
-      const char *c = env + 1;
-      for (int i = 0; i < 4 && *c; i++) {
-        fm[i] = atoi(c);
-        while (*c && *c != ',') c++;
-        if (*c == ',') c++;
-      }
-    }
-    Group Gt = G;  // the first tune_runs runs
-    Gt.nruns = G.tune_runs;
-    const int io[3] = {SLOT_WORK + SNX, SLOT_WORK + SNY, SLOT_WORK + SNZ};
-    const ColJobs jx = jobs_map(io, io, 3);
-    ColJobs jm = jx;
-    jm.masked = 1;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    cudaError_t e = cudaEventCreate(&e0);
-    if (e == cudaSuccess) e = cudaEventCreate(&e1);
-    if (e == cudaSuccess)
-      e = time_cands<0, false>(Gt, st, jx, e0, e1, force, fm[0], rec);
-    if (e == cudaSuccess)
-      e = time_cands<1, false>(Gt, st, jobs_pass_b(false), e0, e1, force, fm[2], rec);
-    if (e == cudaSuccess) e = time_cands<1, true>(Gt, st, jm, e0, e1, force, fm[3], rec);
-    if (e == cudaSuccess) e = time_cands<0, true>(Gt, st, jx, e0, e1, force, fm[1], rec);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
-    if (e == cudaSuccess) tune_cache[G.tune_runs] = rec;
-    memcpy(G.pick, rec.pick, sizeof G.pick);
-    *ran = true;
-    return e;
-  }
-  // text description of the schedules chosen for G
-  static std::string schedule(const Group &G) {
-    std::string out;
-    TuneRec rec{};
-    memcpy(rec.pick, G.pick, sizeof rec.pick);
-    {
-      std::lock_guard<std::mutex> lock(tune_mu);
-      auto it = tune_cache.find(G.tune_runs);
-      if (it != tune_cache.end()) rec = it->second;
-    }
-    if (G.tune_runs > 1) out = "timed on " + std::to_string(G.tune_runs) + " runs: ";
-    const char *name[2][2] = {{"x inverse", "x forward"}, {"y inverse", "y forward"}};
-    char buf[160];
-    for (int a = 0; a < 2; a++)
-      for (int f = 0; f < 2; f++) {
-        const int n = a == 0 ? Cands<0>::n : Cands<1>::n;
-        const int *m = a == 0 ? Cands<0>::m : Cands<1>::m;
-        const int k = rec.pick[a][f];
-        snprintf(buf, sizeof buf, "%scolumn pass %s: min blocks/SM %d of {",
-                 (a == 0 && f == 0) ? "" : "; ", name[a][f], m[k]);
-        out += buf;
-        for (int i = 0; i < n; i++) {
-          snprintf(buf, sizeof buf, "%s%d: %.4f ms", i ? ", " : "", m[i], (double)rec.ms[a][f][i]);
-          out += buf;
-        }
-        out += "}";
-      }
-    return out;
-  }
-
-  template <int KIND>
-  static void zpass(const Group &G, cudaStream_t st, C *work, R *stale, R invn3) {
-    k_zstage<R, N, KIND><<<zsgrid<KIND>(G.nruns), ZC<R, N, KIND>::THREADS, ZS_SMEM<KIND>, st>>>(
-        work, stale, tw(G), G.g, invn3);
-  }
-  // the z pass of RK stage s of one run (the first stage's or the middle
-  // stages' form), keeping the real velocity and vorticity in keep[6][n^3]
-  static void zpass_keep(const Group &G, cudaStream_t st, int s, R *keep) {
-    if constexpr (ZKEEP) {
-      C *work = slot(G, SLOT_WORK);
-      const R invn3 = (R)(1.0 / (double)G.g.nreal);
-      if (s == 0)
-        k_zstage_keep<R, N, 0><<<zsgrid<0>(1), ZC<R, N, 0>::THREADS, ZS_SMEM<0>, st>>>(
-            work, (R *)G.stale, tw(G), G.g, invn3, keep);
-      else
-        k_zstage_keep<R, N, 1><<<zsgrid<1>(1), ZC<R, N, 1>::THREADS, ZS_SMEM<1>, st>>>(
-            work, (R *)G.stale, tw(G), G.g, invn3, keep);
-    }
-  }
-
-  static C *slot(const Group &G, int s) { return (C *)G.S + (long long)s * G.g.slot; }
-  static const C *tw(const Group &G) { return (const C *)G.tw; }
-
-  template <int AXIS, bool FWD>
-  static void colpass_io(const Group &G, cudaStream_t st, const C *in, C *out, const ColJobs &jobs,
-                         int nruns) {
-    // a masked pass covers the tiles holding kz <= kcut
-    const int tiles = jobs.masked ? G.g.kcut / CW<AXIS> + 1 : G.g.nfp / CW<AXIS>;
-    dim3 grid(tiles, N, jobs.njobs * nruns);
-    colkern<AXIS, FWD>(G)<<<grid, CT<AXIS>, COL_SMEM<AXIS>, st>>>(in, out, tw(G), G.g, jobs);
-  }
-  template <int AXIS, bool FWD>
-  static void colpass(const Group &G, cudaStream_t st, const ColJobs &jobs) {
-    colpass_io<AXIS, FWD>(G, st, (C *)G.S, (C *)G.S, jobs, G.nruns);
-  }
-
-  static dim3 zgrid(int nfields) { return dim3((N * N) / ZCfg<N>::LINES, nfields); }
-  template <int KIND>
-  static dim3 zsgrid(int nruns) {
-    return dim3((N * N + ZC<R, N, KIND>::LINES - 1) / ZC<R, N, KIND>::LINES, nruns);
-  }
-
-  static XArgs<R> xargs(const Group &G, int s) {
-    return XArgs<R>{slot(G, SLOT_SA), slot(G, SLOT_RK), slot(G, SLOT_WORK),
-                    (s == 3 && (G.flags & DNS_FLAG_PRESSURE)) ? slot(G, SLOT_P) : nullptr, G.coef};
-  }
-  static dim3 xgrid(const Group &G) { return dim3((G.g.nf + X::W - 1) / X::W, N, G.nruns); }
-
-  // Kernel `k` (K_B..K_X) of RK stage `s` for all runs of G, or with s < 0
-  // the x transform of the state a step starts from: what it runs, its job
-  // table or arguments, and its work items (the launch grid, threads and
-  // shared memory of one block).  The standalone launches (stage_kernel) and
-  // the persistent ensemble kernel's plan are both made from it.
-  static PPhase<R> describe(const Group &G, int s, int k) {
-    const Geo &g = G.g;
-    PPhase<R> P{};
-    P.gz = 1;
-    if (k == K_B || k == K_D) {
-      P.kind = PK_COL;
-      P.fwd = k == K_D;
-      if (k == K_B) {
-        P.jobs = jobs_pass_b(s == 0);
-      } else {
-        // y forward, in place on the three N slots; only the modes inside
-        // the 2/3 rule are computed and stored
-        const int io[3] = {SLOT_WORK + SNX, SLOT_WORK + SNY, SLOT_WORK + SNZ};
-        P.jobs = jobs_map(io, io, 3);
-        P.jobs.masked = 1;
-      }
-      // a masked pass covers the tiles holding kz <= kcut
-      constexpr int cw = CW<1>;
-      P.gx = P.jobs.masked ? g.kcut / cw + 1 : g.nfp / cw;
-      P.gy = N;
-      P.gz = P.jobs.njobs * G.nruns;
-      P.tpi = CT<1>;
-      P.smem = (int)COL_SMEM<1>;
-    } else if (k == K_C) {
-      P.kind = PK_Z;
-      P.sub = s == 0 ? 0 : s < 3 ? 1 : 2;
-      const int lines = P.sub == 0 ? ZC<R, N, 0>::LINES : P.sub == 1 ? ZC<R, N, 1>::LINES
-                                                                      : ZC<R, N, 2>::LINES;
-      P.gx = (N * N + lines - 1) / lines;
-      P.gy = G.nruns;
-      P.tpi = ZC<R, N, 0>::THREADS;
-      P.smem = (int)(P.sub == 0 ? ZS_SMEM<0> : P.sub == 1 ? ZS_SMEM<1> : ZS_SMEM<2>);
-    } else {
-      P.kind = PK_X;
-      P.sub = s;
-      P.xa = xargs(G, s);
-      const dim3 grid = xgrid(G);
-      P.gx = grid.x;
-      P.gy = grid.y;
-      P.gz = grid.z;
-      P.tpi = X::THREADS;
-      P.smem = (int)XS_SMEM;
-    }
-    return P;
-  }
-
-  template <int ST, bool TAIL>
-  static void xpass(const Group &G, cudaStream_t st) {
-    k_xstage<R, N, ST, TAIL>
-        <<<xgrid(G), X::THREADS, XS_SMEM, st>>>(xargs(G, ST), tw(G), G.g);
-  }
-
-  // kernel `k` (K_B..K_X) of RK stage `s`, all runs of G; `tail`: the last
-  // stage's x pass also transforms the new state for the next step
-  static void stage_kernel(const Group &G, cudaStream_t st, int s, int k, bool tail) {
-    const Geo &g = G.g;
-    C *work = slot(G, SLOT_WORK);
-    R *stale = (R *)G.stale;
-    const R invn3 = (R)(1.0 / (double)g.nreal);
-    if (k == K_X) {
-      if (s < 0)
-        xpass<-1, true>(G, st);
-      else if (s == 0)
-        xpass<0, true>(G, st);
-      else if (s == 1)
-        xpass<1, true>(G, st);
-      else if (s == 2)
-        xpass<2, true>(G, st);
-      else if (tail)
-        xpass<3, true>(G, st);
-      else
-        xpass<3, false>(G, st);
-      return;
-    }
-    const PPhase<R> P = describe(G, s, k);
-    if (P.kind == PK_COL) {
-      ColFn f = P.fwd ? colkern<1, true>(G) : colkern<1, false>(G);
-      f<<<dim3(P.gx, P.gy, P.gz), P.tpi, P.smem, st>>>((C *)G.S, (C *)G.S, tw(G), g, P.jobs);
-    } else if (P.sub == 0) {
-      zpass<0>(G, st, work, stale, invn3);
-    } else if (P.sub == 1) {
-      zpass<1>(G, st, work, stale, invn3);
-    } else {
-      zpass<2>(G, st, work, stale, invn3);
-    }
-  }
-
-  // this group's part of the persistent ensemble kernel's plan
-  static void plan_group(const Group &G, PGroup<R> &pg) {
-    pg.n = N;
-    pg.g = G.g;
-    pg.S = (C *)G.S;
-    pg.work = slot(G, SLOT_WORK);
-    pg.stale = (R *)G.stale;
-    pg.tw = tw(G);
-    pg.invn3 = (R)(1.0 / (double)G.g.nreal);
-    pg.ph[0] = describe(G, -1, K_X);
-    for (int s = 0; s < 4; s++)
-      for (int k = 0; k < KERNELS_PER_STAGE; k++)
-        pg.ph[1 + s * KERNELS_PER_STAGE + k] = describe(G, s, k);
-  }
-
-  // the x transform of the state, which a step starts from
-  static void first(const Group &G, cudaStream_t st) { stage_kernel(G, st, -1, K_X, true); }
-  static void step(const Group &G, cudaStream_t st, bool tail) {
-    for (int s = 0; s < 4; s++)
-      for (int k = 0; k < KERNELS_PER_STAGE; k++) stage_kernel(G, st, s, k, tail);
-  }
-
-  // forward transform of the three stale real slots into SA (one run)
-  static void forward(const Group &G, cudaStream_t st) {
-    k_zr2c<R, N><<<zgrid(3), ZCfg<N>::THREADS, Z_SMEM, st>>>((const R *)G.stale,
-                                                              slot(G, SLOT_WORK), tw(G), G.g);
-    const int w3[3] = {SLOT_WORK + 0, SLOT_WORK + 1, SLOT_WORK + 2};
-    const int sa[3] = {SLOT_SA + 0, SLOT_SA + 1, SLOT_SA + 2};
-    colpass<1, true>(G, st, jobs_map(w3, w3, 3));
-    colpass<0, true>(G, st, jobs_map(w3, sa, 3));
-  }
-
-  // c2r(X) / n^3 of SA (and P) into realbuf [4][n^3] float64 (one run)
-  static void backward(const Group &G, cudaStream_t st, int nfields) {
-    const int in[4] = {SLOT_SA + 0, SLOT_SA + 1, SLOT_SA + 2, SLOT_P};
-    const int w4[4] = {SLOT_WORK + 0, SLOT_WORK + 1, SLOT_WORK + 2, SLOT_WORK + 3};
-    colpass<0, false>(G, st, jobs_map(in, w4, nfields));
-    colpass<1, false>(G, st, jobs_map(w4, w4, nfields));
-    k_zc2r<R, N><<<zgrid(nfields), ZCfg<N>::THREADS, Z_SMEM, st>>>(
-        slot(G, SLOT_WORK), G.realbuf, tw(G), G.g, 1.0 / (double)G.g.nreal);
-  }
-
-  // c2r of K spectral fields (in + in_slots[f] * slot) into out[f * nreal],
-  // scaled (one run; uses the work slots)
-  static void c2r_fields(const Group &G, cudaStream_t st, const C *in, const int *in_slots, int K,
-                         double *out, double scale) {
-    C *wk = slot(G, SLOT_WORK);
-    ColJobs j1 = jobs_empty(K), j2 = jobs_empty(K);
-    for (int f = 0; f < K; f++) {
-      j1.in_slot[f] = in_slots[f];
-      j1.out_slot[f] = f;
-      j2.in_slot[f] = f;
-      j2.out_slot[f] = f;
-    }
-    colpass_io<0, false>(G, st, in, wk, j1, 1);
-    colpass_io<1, false>(G, st, wk, wk, j2, 1);
-    k_zc2r<R, N><<<zgrid(K), ZCfg<N>::THREADS, Z_SMEM, st>>>(wk, out, tw(G), G.g, scale);
-  }
-  // r2c of K real fields in[f * nreal] into spectral out + out_slots[f] * slot
-  static void r2c_fields(const Group &G, cudaStream_t st, const R *in, int K, C *out,
-                         const int *out_slots) {
-    C *wk = slot(G, SLOT_WORK);
-    ColJobs j1 = jobs_empty(K), j2 = jobs_empty(K);
-    for (int f = 0; f < K; f++) {
-      j1.in_slot[f] = f;
-      j1.out_slot[f] = out_slots[f];
-      j2.in_slot[f] = f;
-      j2.out_slot[f] = f;
-    }
-    k_zr2c<R, N><<<zgrid(K), ZCfg<N>::THREADS, Z_SMEM, st>>>(in, wk, tw(G), G.g);
-    colpass_io<1, true>(G, st, wk, wk, j2, 1);
-    colpass_io<0, true>(G, st, wk, out, j1, 1);
-  }
-
-  // energy / enstrophy sums of every run into diag_out[run]
-  static void diag(const Group &G, cudaStream_t st) {
-    k_diag<256, C><<<dim3(G.diag_blocks, G.nruns), 256, 0, st>>>(slot(G, SLOT_SA), G.g, G.diag_part);
-    k_diag_final<256><<<G.nruns, 256, 0, st>>>(G.diag_part, G.diag_blocks, G.diag_out);
-  }
-};
 
 template <class F>
 bool dispatch_n(int prec, long n, F &&f) {
@@ -970,7 +448,7 @@ int set_coef(const Group &G, cudaStream_t st, const double *nu, const double *dt
 // reversed step; lambda of dU_s; two transform triples)
 enum { X_LA = 0, X_LB = 3, X_LDU = 6, X_T1 = 9, X_T2 = 12, NX = 15 };
 // real work triples (in units of n^3 fields)
-enum { RE_U = 0, RE_OM = 3, RE_LN = 6, RE_LU = 9, RE_LOM = 12, RE_LSTALE = 15, NRE = 18 };
+enum { RE_LN = 0, RE_LU = 3, RE_LOM = 6, RE_LSTALE = 9, NRE = 12 };
 
 struct Adj {
   Group G;
@@ -982,7 +460,7 @@ struct Adj {
   char *snap_sp = nullptr;   // [S][3][slot]
   char *snap_re = nullptr;   // [S][3][n^3], storage real type
   char *keep = nullptr;      // [4][6][n^3], storage real type: the real velocity and
-                             // vorticity of each RK stage, where the z pass keeps them
+                             // vorticity of each RK stage
   double4 *part = nullptr, *acc_nu = nullptr;
   int nblocks = 0;
   double nu = 0, dt = 0;
@@ -1023,29 +501,14 @@ struct AdjOps {
     const int t3[3] = {0, 1, 2};
     const StageIn<C> Us = stage_input(A, s);
     const unsigned pb = pblocks(A);
-    if constexpr (!O::ZKEEP) {  // the velocity and vorticity of the stage, again
-      k_stage_input<C><<<pb, 256, 0, A.st>>>(Us, A.X<C>(X_T2), g);
-      if (s > 0) O::c2r_fields(G, A.st, A.X<C>(X_T2), t3, 3, A.Rf(RE_U), a);
-      k_curl<C><<<pb, 256, 0, A.st>>>(A.X<C>(X_T2), A.X<C>(X_T1), g);
-      O::c2r_fields(G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_OM), a);
-    }
     k_adj_lamN<C><<<pb, 256, 0, A.st>>>(A.X<C>(X_LDU), A.X<C>(X_T1), g, A.dt);
     O::c2r_fields(G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_LN), 1.0);
     const double *lso = s == 3 ? A.Rf(RE_LSTALE) : nullptr;
     const unsigned cb = conv_blocks(g.nreal);
     // stage 0 reads the stale velocity (main.c:344), the step's input one
-    if constexpr (O::ZKEEP) {  // kept by the z pass of the forward stage
-      const R *u = s > 0 ? A.K<R>(s, 0) : (const R *)G.stale;
-      k_adj_cross<R, R, R><<<cb, 256, 0, A.st>>>(u, A.K<R>(s, 3), A.Rf(RE_LN), lso,
-                                                 A.Rr<R>(RE_LU), A.Rr<R>(RE_LOM), g.nreal);
-    } else if (s > 0) {
-      k_adj_cross<double, double, R><<<cb, 256, 0, A.st>>>(
-          A.Rf(RE_U), A.Rf(RE_OM), A.Rf(RE_LN), lso, A.Rr<R>(RE_LU), A.Rr<R>(RE_LOM), g.nreal);
-    } else {
-      k_adj_cross<R, double, R><<<cb, 256, 0, A.st>>>((const R *)G.stale, A.Rf(RE_OM),
-                                                      A.Rf(RE_LN), lso, A.Rr<R>(RE_LU),
-                                                      A.Rr<R>(RE_LOM), g.nreal);
-    }
+    const R *u = s > 0 ? A.K<R>(s, 0) : (const R *)G.stale;
+    k_adj_cross<R, R, R><<<cb, 256, 0, A.st>>>(u, A.K<R>(s, 3), A.Rf(RE_LN), lso, A.Rr<R>(RE_LU),
+                                               A.Rr<R>(RE_LOM), g.nreal);
     O::r2c_fields(G, A.st, A.Rr<R>(RE_LOM), 3, A.X<C>(X_T1), t3);
     if (s > 0) O::r2c_fields(G, A.st, A.Rr<R>(RE_LU), 3, A.X<C>(X_T2), t3);
     k_adj_collect<256, C><<<pb, 256, 0, A.st>>>(
@@ -1064,24 +527,19 @@ struct AdjOps {
   // other buffer, which becomes A.lhat).  The forward stages 0-2 run again
   // to recover the stage inputs U_1..U_3 (stage 3's output is not needed);
   // the step's state (SA, stale) is left in place for stage 0's adjoint.
-  // Where the z pass can keep its real velocity and vorticity, every stage's
-  // z pass (stage 3's too, after its y pass; without its stale store) keeps
-  // them for the transposed stage.
+  // Every stage's z pass (stage 3's too, without its stale store) keeps its
+  // real velocity and vorticity for the transposed stage.
   static int step(Adj &A) {
     const Group &G = A.G;
     const Geo &g = G.g;
     int r;
     O::first(G, A.st);
-    for (int s = 0; s < 4; s++) {
-      if (!O::ZKEEP && s == 3) break;
-      for (int k = 0; k < KERNELS_PER_STAGE; k++) {
-        if (s == 3 && k > K_C) break;
-        if (O::ZKEEP && k == K_C)
-          O::zpass_keep(G, A.st, s, A.K<R>(s, 0));
-        else
-          O::stage_kernel(G, A.st, s, k, true);
+    for (int s = 0; s < 4; s++)
+      for (int q = 0; q < O::kernels(G); q++) {
+        const int k = O::kernel(G, q);
+        if (s == 3 && (k == K_D || k == K_X)) break;
+        O::stage_kernel(G, A.st, s, k, true, A.K<R>(s, 0));
       }
-    }
     const int lo = A.lhat, li = A.lhat == X_LA ? X_LB : X_LA;
     const C *lacc = A.X<C>(lo);  // lambda of the accumulator: that of the step output
     // lambda_dU of stage 3 = a_3 lambda_acc
@@ -1442,8 +900,25 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
     c->cur_nu = nu;
     c->cur_dt = dt;
   }
-  // launches of a step: the x transform of the state, then B, C, D, X a stage
-  const int K = c->kernels_per_step, L = 1 + 4 * KERNELS_PER_STAGE;
+  // the launches of a step: the x transform of the state, then each stage's
+  // kernels, with the passes each of them runs (the x pass a stage's E1 and
+  // E2 and, except in the last, the next one's A)
+  const int K = c->kernels_per_step;
+  struct Launch {
+    int s, k, first, count;
+  };
+  std::vector<Launch> launches{{-1, K_X, 0, 1}};
+  dispatch(c->grp, [&](auto ops) {
+    using O = decltype(ops);
+    for (int s = 0; s < 4; s++)
+      for (int q = 0; q < O::kernels(c->grp); q++) {
+        const int k = O::kernel(c->grp, q), p0 = s * PASSES_PER_STAGE;
+        launches.push_back(k == K_X    ? Launch{s, k, p0 + 4, s < 3 ? 3 : 2}
+                           : k == K_YZ ? Launch{s, k, p0 + 1, 3}
+                                       : Launch{s, k, p0 + 1 + k, 1});
+      }
+  });
+  const int L = (int)launches.size();
   // destroyed on every return path, the early ones of CK included
   struct Events {
     std::vector<cudaEvent_t> v;
@@ -1460,10 +935,8 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
   for (long s = 0; s < nsteps && st == DNS_OK; s++) {
     CK(cudaEventRecord(ev[0], c->stream));
     for (int k = 0; k < L; k++) {
-      const int q = k - 1;
       dispatch(c->grp, [&](auto ops) {
-        decltype(ops)::stage_kernel(c->grp, c->stream, k == 0 ? -1 : q / KERNELS_PER_STAGE,
-                                    k == 0 ? (int)K_X : q % KERNELS_PER_STAGE, false);
+        decltype(ops)::stage_kernel(c->grp, c->stream, launches[k].s, launches[k].k, false);
       });
       CK(cudaEventRecord(ev[k + 1], c->stream));
     }
@@ -1472,21 +945,7 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
     for (int k = 0; k < L; k++) {
       float t = 0.f;
       CK(cudaEventElapsedTime(&t, ev[k], ev[k + 1]));
-      if (k == 0) {
-        ms[0] += t;
-        continue;
-      }
-      double *row = ms + (k - 1) / KERNELS_PER_STAGE * PASSES_PER_STAGE;
-      const int kern = (k - 1) % KERNELS_PER_STAGE;
-      if (kern != K_X) {
-        row[1 + kern] += t;
-      } else {  // E1 and E2 of this stage and, except after the last, A of the next
-        const bool tail = k + 1 < L;
-        const double share = t / (tail ? 3.0 : 2.0);
-        row[4] += share;
-        row[5] += share;
-        if (tail) row[PASSES_PER_STAGE] += share;
-      }
+      for (int p = 0; p < launches[k].count; p++) ms[launches[k].first + p] += t / launches[k].count;
     }
   }
   for (int k = 0; k < K; k++) ms[k] /= (double)nsteps;
@@ -1759,8 +1218,8 @@ int dns_ens_set_params(dns_ens *e, const double *nu, const double *dt) {
   return DNS_OK;
 }
 
-// one graph: a fork per size group (its own stream), each group's 16
-// batched kernels, then a join
+// one graph: a fork per size group (its own stream), each group's
+// batched kernels (16, or 8 where Ops::plane), then a join
 static int ens_build_graph(dns_ens *e, bool tail, cudaGraphExec_t *out) {
   if (*out) return DNS_OK;
   cudaGraph_t gr;
@@ -1920,11 +1379,8 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
     const size_t keep_b = (size_t)24 * g.nreal * A.G.rsize;
     const size_t part_b = (size_t)(A.nblocks + 1) * sizeof(double4);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    bool zkeep = false;
-    dispatch(A.G, [&](auto ops) { zkeep = decltype(ops)::ZKEEP; });
-    const size_t keep_a = zkeep ? al(keep_b) : 0;
     cudaError_t e = dev_malloc((void **)&A.arena,
-                               al(sp_b) + al(re_b) + al(ssp_b) + al(sre_b) + keep_a + al(part_b));
+                               al(sp_b) + al(re_b) + al(ssp_b) + al(sre_b) + al(keep_b) + al(part_b));
     if (e != cudaSuccess) {
       A.arena = nullptr;
       r = fail(DNS_ERR_NOMEM, cudaGetErrorString(e), __FILE__, __LINE__);
@@ -1934,10 +1390,7 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
       A.re = (double *)p; p += al(re_b);
       A.snap_sp = p; p += al(ssp_b);
       A.snap_re = p; p += al(sre_b);
-      if (zkeep) {
-        A.keep = p;
-        p += keep_a;
-      }
+      A.keep = p; p += al(keep_b);
       A.part = (double4 *)p;
       A.acc_nu = A.part + A.nblocks;
       e = cudaMemsetAsync(A.arena, 0, al(sp_b) + al(re_b), A.st);

@@ -1,6 +1,7 @@
-// ens_persistent.cu -- the persistent ensemble kernel (persistent.cuh) and
-// its launch entry points, in a translation unit of their own: the kernel
-// inlines every pass body of every grid size it supports.
+// ens_kernel.cuh -- the persistent ensemble kernel (persistent.cuh) and its
+// launch entry points, included by one translation unit per precision: the
+// kernel inlines every pass body of every grid size it supports.
+#pragma once
 #define DNSB_PERSISTENT_KERNELS
 #include "persistent.cuh"
 
@@ -30,17 +31,5 @@ cudaError_t p_launch(int grid, size_t smem, cudaStream_t st, const PPlan<R> *pla
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k_ens_step<R>, plan, sy, wait_ns);
 }
-
-cudaError_t p_barrier_selftest(PSync *sy, cudaStream_t st, unsigned long long wait_ns) {
-  k_barrier_selftest<<<2, 32, 0, st>>>(sy, wait_ns);
-  return cudaGetLastError();
-}
-
-template cudaError_t p_prepare<float>(size_t, int *);
-template cudaError_t p_prepare<double>(size_t, int *);
-template cudaError_t p_launch<float>(int, size_t, cudaStream_t, const PPlan<float> *, PSync *,
-                                     unsigned long long);
-template cudaError_t p_launch<double>(int, size_t, cudaStream_t, const PPlan<double> *, PSync *,
-                                      unsigned long long);
 
 }  // namespace dnsb

@@ -51,6 +51,19 @@ template <class C>
 __device__ __forceinline__ C czero() {
   return cmk<C>(sc<C>(0), sc<C>(0));
 }
+// Where the compiler could choose which product to contract into an addition
+// (a b + c d), or whether to contract one into a following butterfly, the
+// roundings are written out: every kernel that inlines the code computes the
+// same bits (one run alone or in a batch, whichever kernels its size and batch
+// take, and the value that the x pass stores and the one it transforms on the
+// spot).
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
+
 template <class C>
 __device__ __forceinline__ C cadd(C a, C b) { return cmk<C>(a.x + b.x, a.y + b.y); }
 template <class C>
@@ -60,12 +73,12 @@ __device__ __forceinline__ C cscale(C a, sc<C> s) { return cmk<C>(a.x * s, a.y *
 // a * b
 template <class C>
 __device__ __forceinline__ C cmul(C a, C b) {
-  return cmk<C>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return cmk<C>(fma_rn(a.x, b.x, mul_rn(-a.y, b.y)), fma_rn(a.x, b.y, mul_rn(a.y, b.x)));
 }
 // a * conj(b)
 template <class C>
 __device__ __forceinline__ C cmulc(C a, C b) {
-  return cmk<C>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+  return cmk<C>(fma_rn(a.x, b.x, mul_rn(a.y, b.y)), fma_rn(a.y, b.x, mul_rn(-a.x, b.y)));
 }
 // multiply by the twiddle w (forward table entry) in the given direction
 template <bool FWD, class C>
@@ -111,9 +124,9 @@ __device__ __forceinline__ C w16(C a) {
     constexpr S s = (S)(q == 0 ? s0 : q == 1 ? c0 : q == 2 ? -s0 : -c0);
     // forward multiplies by (c - i s), backward by (c + i s)
     if constexpr (FWD)
-      return cmk<C>(a.x * c + a.y * s, a.y * c - a.x * s);
+      return cmk<C>(fma_rn(a.x, c, mul_rn(a.y, s)), fma_rn(a.y, c, mul_rn(-a.x, s)));
     else
-      return cmk<C>(a.x * c - a.y * s, a.y * c + a.x * s);
+      return cmk<C>(fma_rn(a.x, c, mul_rn(-a.y, s)), fma_rn(a.y, c, mul_rn(a.x, s)));
   }
 }
 

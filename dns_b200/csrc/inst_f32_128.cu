@@ -1,0 +1,6 @@
+#include "ops.cuh"
+
+// the kernels of these sizes (instances.cuh): taking setup's address compiles
+// every kernel it prepares
+extern cudaError_t (*const dnsb_inst_f32_128[])();
+cudaError_t (*const dnsb_inst_f32_128[])() = {&Ops<float, 128>::setup};

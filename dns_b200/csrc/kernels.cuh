@@ -17,7 +17,7 @@
 // The same slot shape holds partially transformed data: after the x pass the
 // first index is x instead of kx, after the y pass the second is y.
 //
-// One RK stage = four kernels:
+// One RK stage = four kernels (two where YZ runs B, C and D in one, n <= 64):
 //   B   y backward  5 slots -> u,v,w, omega_z = dv/dx - du/dy, dw/dx, dw/dy
 //   C   z pass      per z line: vorticity from the 6 slots, u and omega to
 //                   real space, N = u x omega, N back to z spectral (stored
@@ -45,6 +45,18 @@ namespace dnsb {
 // in it has been read, and D and X take N from there.
 enum { SU = 0, SV = 1, SDWDY = 2, SOMZ = 3, SDWDX = 4, SW = 5, NWORK = 6 };
 enum { SNX = 0, SNY = 1, SNZ = 2 };
+
+// Loads that leave no line in L1: where shared memory leaves little of it, the
+// lines reserved for loads in flight bound how many there are.
+template <class C>
+__device__ __forceinline__ C ldcg(const C *p) {
+  return __ldcg(p);
+}
+// 16-byte asynchronous copy from global to shared memory, past L1
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
 
 struct Geo {
   int n, nf, nfp;
@@ -186,7 +198,7 @@ __device__ __forceinline__ void colpass_body(const cx<R> *__restrict__ in, cx<R>
 #pragma unroll
       for (int e = 0; e < E; e++) {
         const R k = (R)kwave(t + T * e, N);
-        v[e] = cmk<C>(-k * v[e].y, k * v[e].x);  // i k f
+        v[e] = cmk<C>(mul_rn(-k, v[e].y), mul_rn(k, v[e].x));  // i k f
       }
     } else if (pass == 0) {
       const C *add = in + (long long)aslot * g.slot + base;
@@ -194,7 +206,7 @@ __device__ __forceinline__ void colpass_body(const cx<R> *__restrict__ in, cx<R>
       for (int e = 0; e < E; e++) {
         const R k = (R)kwave(t + T * e, N);
         const C a = ok ? add[(t + T * e) * rs] : czero<C>();
-        v[e] = cmk<C>(a.x + k * v[e].y, a.y - k * v[e].x);  // add - i k f
+        v[e] = cmk<C>(fma_rn(k, v[e].y, a.x), fma_rn(-k, v[e].x, a.y));  // add - i k f
       }
     }
     line_fft<N, Plan<N>, FWD>(v, t, st, xb, ColIdx<W>{p}, sync);
@@ -445,34 +457,31 @@ struct ZC {
   static constexpr int E = P::E;
   static constexpr int T = N / E;                 // threads per line
   static constexpr int M = N / 2;
-  // FP64 with 16 values per thread (S2) and FP32: the pairs run in the
-  // order (u, omega_y), (v, omega_x), (w, omega_z), so that N_z is complete
-  // after the second and goes through its forward FFT and out before the
-  // third; N_x and N_y are then formed in place in the FFT registers.  At
-  // most two fields beyond the FFT's own values are live: FP64 keeps (u,
-  // omega_y) in shared memory and (v, omega_x) in registers (128-thread
-  // blocks of 8 lines, 2 per SM, which build the stage twiddles once for 8
-  // lines: 1-10 % faster than 64-thread blocks at 4 per SM; capping the
-  // registers for more blocks measured slower); FP32 keeps both pairs in
-  // registers (128 of them; 512^3 in 256-thread blocks at 2 per SM, 10 %
-  // faster there than 128-thread blocks at 4, 1 % slower at 256^3).  The
-  // first stage reads the stale velocity where it needs it.
+  // The pairs run in the order (u, omega_y), (v, omega_x), (w, omega_z), so
+  // that N_z is complete after the second and goes through its forward FFT
+  // and out before the third; N_x and N_y are then formed in place in the FFT
+  // registers.  At most two fields beyond the FFT's own values are live: FP64
+  // with 16 values per thread (S2) keeps (u, omega_y) in shared memory and
+  // (v, omega_x) in registers (128-thread blocks of 8 lines, 2 per SM, which
+  // build the stage twiddles once for 8 lines: 1-10 % faster than 64-thread
+  // blocks at 4 per SM; capping the registers for more blocks measured
+  // slower); with 8 values, and in FP32, both pairs are in registers (128 of
+  // them; FP32 512^3 in 256-thread blocks at 2 per SM, 10 % faster there than
+  // 128-thread blocks at 4, 1 % slower at 256^3).  The first stage reads the
+  // stale velocity where it needs it.
   static constexpr bool S2 = sizeof(R) == 8 && E >= 16;
   static constexpr bool F32 = sizeof(R) == 4;
   static constexpr int WANT = (F32 && N > 256) ? 256 : 128;
   static constexpr int THREADS = (N * N * T) < WANT ? (N * N * T) : WANT;
   static constexpr int LINES = THREADS / T;
-  static constexpr int MINB = S2 ? 2 : F32 ? (N > 256 ? 2 : 4) : 3;  // blocks per SM
+  static constexpr int MINB = S2 ? 2 : (F32 && N > 256) ? 2 : 4;  // blocks per SM
   static constexpr int PADSH = (E >= 16) ? 4 : 3;
   static constexpr int XB = N + (N >> PADSH);     // padded exchange buffer (complex)
   // stage twiddle entries held (even, so the exchange buffers stay 16-byte
   // aligned)
   static constexpr int TWN = (StageTw<P>::SIZE + 1) / 2 * 2 > 2 ? (StageTw<P>::SIZE + 1) / 2 * 2 : 2;
-  // staged scalars per line: S2 none (first stage) or (u, omega_y); FP32
-  // none; FP64 with 8 values per thread none (middle stage) or u, v, w,
-  // N_y, N_z
-  static constexpr int STASH =
-      S2 ? (KIND == 0 ? 0 : 2 * N) : ((KIND == 1 || F32) ? 0 : 5 * N);
+  // staged scalars per line: S2 none (first stage) or (u, omega_y)
+  static constexpr int STASH = S2 && KIND != 0 ? 2 * N : 0;
   static constexpr size_t SMEM =
       (size_t)(TWN + LINES * XB) * sizeof(cx<R>) + (size_t)LINES * STASH * sizeof(R);
 };
@@ -584,29 +593,10 @@ __device__ __forceinline__ void zfwd_z(cx<R> (&y)[ZC<R, N, KIND>::E], int t, con
     if (k <= KZ && ok) oW[k] = y[e];
   }
 }
-// both, from N held in registers (the stages that complete N at the end)
-template <class R, int N, int KIND, class Idx, class Sync>
-__device__ __forceinline__ void zstage_forward(cx<R> (&y)[ZC<R, N, KIND>::E],
-                                               const R (&nx)[ZC<R, N, KIND>::E],
-                                               const R (&ny)[ZC<R, N, KIND>::E],
-                                               const R (&nz)[ZC<R, N, KIND>::E], int t,
-                                               const cx<R> *tw, cx<R> *xb, Idx idx, Sync sync,
-                                               cx<R> *row, const Geo &g, bool ok) {
-  using C = cx<R>;
-  constexpr int E = ZC<R, N, KIND>::E;
-#pragma unroll
-  for (int e = 0; e < E; e++) y[e] = cmk<C>(nx[e], ny[e]);
-  zfwd_xy<R, N, KIND>(y, t, tw, xb, idx, sync, row, g, ok);
-#pragma unroll
-  for (int e = 0; e < E; e++) y[e] = cmk<C>(nz[e], R(0));
-  zfwd_z<R, N, KIND>(y, t, tw, xb, idx, sync, row, g, ok);
-}
-
 // One block of the z pass: Z::LINES lines starting at line b.x * LINES of
 // run b.y (block-wide barriers through `bsync`, which lines of more than 32
-// threads also use between FFT stages).  KEEP (the pair orders of S2 and
-// FP32 only): also store the real velocity and vorticity the pass forms in
-// keep[f][n^3], f = u, v, w, omega_x, omega_y, omega_z of the run (the
+// threads also use between FFT stages).  KEEP: also store the real velocity
+// and vorticity the pass forms in keep[f][n^3], f = u, v, w, omega_x, omega_y, omega_z of the run (the
 // first stage: the vorticity only), for the discrete adjoint.
 template <class R, int N, int KIND, bool KEEP = false, class BSync>
 __device__ __forceinline__ void zstage_body(cx<R> *__restrict__ work, R *__restrict__ stale,
@@ -637,11 +627,11 @@ __device__ __forceinline__ void zstage_body(cx<R> *__restrict__ work, R *__restr
   auto ld = [&](const C *p, int s) -> C { return ok ? p[s] : czero<C>(); };
   auto f_ox = [&](int s) -> C {  // omega_x = dw/dy - i kz v
     const C a = ld(pDWDY, s), v = ld(pV, s);
-    return cmk<C>(a.x + (R)s * v.y, a.y - (R)s * v.x);
+    return cmk<C>(fma_rn((R)s, v.y, a.x), fma_rn(-(R)s, v.x, a.y));
   };
   auto f_oy = [&](int s) -> C {  // omega_y = i kz u - dw/dx
     const C u = ld(pU, s), b = ld(pDWDX, s);
-    return cmk<C>(-(R)s * u.y - b.x, (R)s * u.x - b.y);
+    return cmk<C>(fma_rn(-(R)s, u.y, -b.x), fma_rn((R)s, u.x, -b.y));
   };
   auto f_oz = [&](int s) -> C {  // omega_z = dv/dx - du/dy
     return ld(pOMZ, s);
@@ -666,232 +656,103 @@ __device__ __forceinline__ void zstage_body(cx<R> *__restrict__ work, R *__restr
   };
 
   C y[E];
-  if constexpr (Z::S2 || Z::F32) {
-    if constexpr (KIND == 0) {
-      // first stage: (omega_x, omega_y) with the stale real velocity read
-      // where it is needed (L1/L2 hits the second time); N_z is complete
-      // after this pair and leaves before (omega_z, 0)
-      auto sv = [&](int f, int e) -> R { return ok ? stale[f * g.nreal + roff + t + T * e] : R(0); };
-      R nx[E], ny[E];
-      ext_pair<R, N, KIND>(y, t, f_ox, f_oy);
-      pf(pOMZ, ROWB);
-      pf(stale + roff, REALB);
-      pf(stale + g.nreal + roff, REALB);
-      pf(stale + 2 * g.nreal + roff, REALB);
-      line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const R ox = y[e].x * invn3, oy = y[e].y * invn3;
-        const R u = sv(0, e), v = sv(1, e), w = sv(2, e);
-        nx[e] = -w * oy;
-        ny[e] = w * ox;
-        y[e] = cmk<C>(u * oy - v * ox, R(0));  // N_z
-        kp(3, e, ox);
-        kp(4, e, oy);
-      }
-      zfwd_z<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
-      ext_pair<R, N, KIND>(y, t, f_oz, f_zero);
-      line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const R oz = y[e].x * invn3;
-        y[e] = cmk<C>(nx[e] + sv(1, e) * oz, ny[e] - sv(0, e) * oz);  // (N_x, N_y)
-        kp(5, e, oz);
-      }
-      zfwd_xy<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
-    } else {
-      // middle and last stages: (u, omega_y), (v, omega_x): N_z = u oy - v ox
-      // leaves; (w, omega_z): N_x = v oz - w oy, N_y = w ox - u oz formed in
-      // place and leave.  The last stage stores the velocity as the next
-      // stale one as it comes.
-      R su[Z::S2 ? 1 : E], soy[Z::S2 ? 1 : E];  // FP32: (u, omega_y) in registers
-      ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
-        const C uu = ld(pU, s), d = ld(pDWDX, s);
-        a = uu;
-        b = cmk<C>(-(R)s * uu.y - d.x, (R)s * uu.x - d.y);  // i kz u - dw/dx
-      });
-      pf(pV, ROWB);
-      pf(pDWDY, ROWB);
-      line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const R u = y[e].x * invn3, oy = y[e].y * invn3;
-        if constexpr (Z::S2) {
-          SU_(0, e) = u;
-          SU_(1, e) = oy;
-        } else {
-          su[e] = u;
-          soy[e] = oy;
-        }
-        if (KIND == 2 && ok) stale[roff + t + T * e] = u;
-        kp(0, e, u);
-        kp(4, e, oy);
-      }
-      auto U_ = [&](int e) -> R { if constexpr (Z::S2) return SU_(0, e); else return su[e]; };
-      auto OY_ = [&](int e) -> R { if constexpr (Z::S2) return SU_(1, e); else return soy[e]; };
-      ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
-        const C vv = ld(pV, s), d = ld(pDWDY, s);
-        a = vv;
-        b = cmk<C>(d.x + (R)s * vv.y, d.y - (R)s * vv.x);  // dw/dy - i kz v
-      });
-      pf(pW, ROWB);
-      pf(pOMZ, ROWB);
-      line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-      R sv_[E], sox[E];
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const R v = y[e].x * invn3, ox = y[e].y * invn3;
-        sv_[e] = v;
-        sox[e] = ox;
-        const R nz = U_(e) * OY_(e);
-        y[e] = cmk<C>(nz - v * ox, R(0));  // N_z
-        if (KIND == 2 && ok) stale[g.nreal + roff + t + T * e] = v;
-        kp(1, e, v);
-        kp(3, e, ox);
-      }
-      zfwd_z<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
-      ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
-        a = ld(pW, s);
-        b = ld(pOMZ, s);
-      });
-      line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const R w = y[e].x * invn3, oz = y[e].y * invn3;
-        const R nx = -w * OY_(e), ny = -U_(e) * oz;
-        y[e] = cmk<C>(nx + sv_[e] * oz, ny + w * sox[e]);  // (N_x, N_y)
-        if (KIND == 2 && ok) stale[2 * g.nreal + roff + t + T * e] = w;
-        kp(2, e, w);
-        kp(5, e, oz);
-      }
-      zfwd_xy<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
-    }
-  } else {
-    // FP64 with 8 values per thread (n <= 64): N in registers, forward
-    // transforms at the end
-    R nx[E], ny[E], nz[E];
-    if (KIND == 0) {
-    // stale real velocity, own points m = t + T e
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const int m = t + T * e;
-#pragma unroll
-      for (int f = 0; f < 3; f++) SU_(f, e) = ok ? stale[f * g.nreal + roff + m] : R(0);
-    }
+  if constexpr (KIND == 0) {
+    // first stage: (omega_x, omega_y) with the stale real velocity read
+    // where it is needed (L1/L2 hits the second time); N_z is complete
+    // after this pair and leaves before (omega_z, 0)
+    auto sv = [&](int f, int e) -> R { return ok ? stale[f * g.nreal + roff + t + T * e] : R(0); };
+    R nx[E], ny[E];
     ext_pair<R, N, KIND>(y, t, f_ox, f_oy);
+    pf(pOMZ, ROWB);
+    pf(stale + roff, REALB);
+    pf(stale + g.nreal + roff, REALB);
+    pf(stale + 2 * g.nreal + roff, REALB);
     line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
 #pragma unroll
     for (int e = 0; e < E; e++) {
       const R ox = y[e].x * invn3, oy = y[e].y * invn3;
-      const R u = SU_(0, e), v = SU_(1, e), w = SU_(2, e);
-      nx[e] = -w * oy;
-      ny[e] = w * ox;
-      nz[e] = u * oy - v * ox;
+      const R u = sv(0, e), v = sv(1, e), w = sv(2, e);
+      nx[e] = mul_rn(-w, oy);
+      ny[e] = mul_rn(w, ox);
+      y[e] = cmk<C>(fma_rn(-v, ox, mul_rn(u, oy)), R(0));  // N_z
+      kp(3, e, ox);
+      kp(4, e, oy);
     }
+    zfwd_z<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
     ext_pair<R, N, KIND>(y, t, f_oz, f_zero);
     line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
 #pragma unroll
     for (int e = 0; e < E; e++) {
       const R oz = y[e].x * invn3;
-      nx[e] += SU_(1, e) * oz;
-      ny[e] -= SU_(0, e) * oz;
+      y[e] = cmk<C>(fma_rn(sv(1, e), oz, nx[e]), fma_rn(-sv(0, e), oz, ny[e]));  // (N_x, N_y)
+      kp(5, e, oz);
     }
-    } else if (KIND == 1) {
-    // Pairs ordered so that every input slot is read once and the cross
-    // product accumulates in registers (FP32 last stage: the velocity is
-    // stored as the next stale one as it comes):
-    //   (u, omega_y): N_z = u oy
-    //   (w, omega_z): N_x = -w oy, N_y = -u oz
-    //   (v, omega_x): N_x += v oz, N_y += w ox, N_z -= v ox
-    R u[E], oy[E];
+    zfwd_xy<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
+  } else {
+    // middle and last stages: (u, omega_y), (v, omega_x): N_z = u oy - v ox
+    // leaves; (w, omega_z): N_x = v oz - w oy, N_y = w ox - u oz formed in
+    // place and leave.  The last stage stores the velocity as the next
+    // stale one as it comes.
+    R su[Z::S2 ? 1 : E], soy[Z::S2 ? 1 : E];  // (u, omega_y) in registers
     ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
       const C uu = ld(pU, s), d = ld(pDWDX, s);
       a = uu;
-      b = cmk<C>(-(R)s * uu.y - d.x, (R)s * uu.x - d.y);  // i kz u - dw/dx
-    });
-    pf(pW, ROWB);
-    pf(pOMZ, ROWB);
-    line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      u[e] = y[e].x * invn3;
-      oy[e] = y[e].y * invn3;
-      nz[e] = u[e] * oy[e];
-      if (KIND == 2 && ok) stale[roff + t + T * e] = u[e];
-    }
-    ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
-      a = ld(pW, s);
-      b = ld(pOMZ, s);
+      b = cmk<C>(fma_rn(-(R)s, uu.y, -d.x), fma_rn((R)s, uu.x, -d.y));  // i kz u - dw/dx
     });
     pf(pV, ROWB);
     pf(pDWDY, ROWB);
     line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-    R w[E], oz[E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      w[e] = y[e].x * invn3;
-      oz[e] = y[e].y * invn3;
-      nx[e] = -w[e] * oy[e];
-      ny[e] = -u[e] * oz[e];
-      if (KIND == 2 && ok) stale[2 * g.nreal + roff + t + T * e] = w[e];
+      const R u = y[e].x * invn3, oy = y[e].y * invn3;
+      if constexpr (Z::S2) {
+        SU_(0, e) = u;
+        SU_(1, e) = oy;
+      } else {
+        su[e] = u;
+        soy[e] = oy;
+      }
+      if (KIND == 2 && ok) stale[roff + t + T * e] = u;
+      kp(0, e, u);
+      kp(4, e, oy);
     }
+    auto U_ = [&](int e) -> R { if constexpr (Z::S2) return SU_(0, e); else return su[e]; };
+    auto OY_ = [&](int e) -> R { if constexpr (Z::S2) return SU_(1, e); else return soy[e]; };
     ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
       const C vv = ld(pV, s), d = ld(pDWDY, s);
       a = vv;
-      b = cmk<C>(d.x + (R)s * vv.y, d.y - (R)s * vv.x);  // dw/dy - i kz v
+      b = cmk<C>(fma_rn((R)s, vv.y, d.x), fma_rn(-(R)s, vv.x, d.y));  // dw/dy - i kz v
+    });
+    pf(pW, ROWB);
+    pf(pOMZ, ROWB);
+    line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
+    R sv_[E], sox[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const R v = y[e].x * invn3, ox = y[e].y * invn3;
+      sv_[e] = v;
+      sox[e] = ox;
+      y[e] = cmk<C>(fma_rn(-v, ox, mul_rn(U_(e), OY_(e))), R(0));  // N_z
+      if (KIND == 2 && ok) stale[g.nreal + roff + t + T * e] = v;
+      kp(1, e, v);
+      kp(3, e, ox);
+    }
+    zfwd_z<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
+    ext_gen<R, N, KIND>(y, t, [&](int s, C &a, C &b) {
+      a = ld(pW, s);
+      b = ld(pOMZ, s);
     });
     line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      const R v = y[e].x * invn3, ox = y[e].y * invn3;
-      nx[e] += v * oz[e];
-      ny[e] += w[e] * ox;
-      nz[e] -= v * ox;
-      if (KIND == 2 && ok) stale[g.nreal + roff + t + T * e] = v;
+      const R w = y[e].x * invn3, oz = y[e].y * invn3;
+      const R nx = mul_rn(-w, OY_(e)), ny = mul_rn(-U_(e), oz);
+      y[e] = cmk<C>(fma_rn(sv_[e], oz, nx), fma_rn(w, sox[e], ny));  // (N_x, N_y)
+      if (KIND == 2 && ok) stale[2 * g.nreal + roff + t + T * e] = w;
+      kp(2, e, w);
+      kp(5, e, oz);
     }
-    } else {
-    // FP64 last stage at 8 values per thread: the velocity is also stored as
-    // the next stale one, so it is staged in shared memory (the register-only
-    // order above spills here)
-    // (u, v)
-    ext_pair<R, N, KIND>(y, t, [&](int s) { return ld(pU, s); }, [&](int s) { return ld(pV, s); });
-    line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      SU_(0, e) = y[e].x * invn3;
-      SU_(1, e) = y[e].y * invn3;
-    }
-    // (w, omega_x)
-    ext_pair<R, N, KIND>(y, t, [&](int s) { return ld(pW, s); }, f_ox);
-    line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const R w = y[e].x * invn3, ox = y[e].y * invn3;
-      SU_(2, e) = w;
-      SU_(3, e) = w * ox;            // partial N_y
-      SU_(4, e) = -SU_(1, e) * ox;   // partial N_z
-    }
-    // (omega_y, omega_z)
-    ext_pair<R, N, KIND>(y, t, f_oy, f_oz);
-    line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
-#pragma unroll
-    for (int e = 0; e < E; e++) {
-      const R oy = y[e].x * invn3, oz = y[e].y * invn3;
-      const R u = SU_(0, e), v = SU_(1, e), w = SU_(2, e);
-      nx[e] = v * oz - w * oy;
-      ny[e] = SU_(3, e) - u * oz;
-      nz[e] = SU_(4, e) + u * oy;
-    }
-    if (KIND == 2 && ok) {
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        const int m = t + T * e;
-#pragma unroll
-        for (int f = 0; f < 3; f++) stale[f * g.nreal + roff + m] = SU_(f, e);
-      }
-    }
-  }
-    zstage_forward<R, N, KIND>(y, nx, ny, nz, t, tw, xb, idx, sync, work + off, g, ok);
+    zfwd_xy<R, N, KIND>(y, t, tw, xb, idx, sync, work + off, g, ok);
   }
 }
 
@@ -904,16 +765,339 @@ __global__ void __launch_bounds__(ZC<R, N, KIND>::THREADS, ZC<R, N, KIND>::MINB)
 }
 
 // The z pass that also keeps the real velocity and vorticity (KEEP above),
-// for the forward recomputation of the discrete adjoint; the pair orders of
-// S2 and FP32 only.
+// for the forward recomputation of the discrete adjoint.
 template <class R, int N, int KIND>
 __global__ void __launch_bounds__(ZC<R, N, KIND>::THREADS, ZC<R, N, KIND>::MINB)
     k_zstage_keep(cx<R> *__restrict__ work, R *__restrict__ stale, const cx<R> *__restrict__ twg,
                   Geo g, R invn3, R *__restrict__ keep) {
-  static_assert(ZC<R, N, KIND>::S2 || ZC<R, N, KIND>::F32, "KEEP needs the S2 or FP32 pair order");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   zstage_body<R, N, KIND, true>(work, stale, twg, g, invn3, launch_blk(), BlockSync{}, smem_raw,
                                 keep);
+}
+
+// ---------------------------------------------------------------------------
+// YZ: for n <= 64 a whole x plane (six fields, ky or y by kz) fits the shared
+// memory of one SM (FP64 n = 64: 217 KB), so the y backward pass, the z pass
+// and the y forward pass of a plane (B, C and D above) run as one kernel:
+// 6.3 slots of traffic a stage instead of 22.3, and two launches fewer.
+//
+// The plane is held as three pairs of fields, (u, dw/dx), (v, dw/dy) and
+// (w, omega_z), a row of a pair being RP complex values: the first field's
+// kz = 0..n/2 from 0, the second's from HP on.  A row of a pair is exactly the
+// exchange buffer of that pair's z transforms (the pair of fields that the
+// two-for-one FFT takes), and a column of a field that of its y transforms,
+// so no transform needs other shared memory.  Every transform runs inside
+// one warp; the block meets twice, between the axes.  The arithmetic is that
+// of colpass_body and zstage_body, bit for bit.
+//
+// Step of n = 16 FP64 0.117 -> 0.047 ms, n = 32 0.086 -> 0.058; 32 runs of
+// 64^3 in FP32 1.67 -> 1.06 ms (the x pass alone had brought 1.40).  At n = 64 it is
+// bound by the shared-memory pipe of the SMs that have a plane: some 2.4 MB a
+// plane in FP64.
+// ---------------------------------------------------------------------------
+template <class R, int N>
+struct YZ {
+  using P = Plan<N>;
+  static constexpr int E = P::E, T = N / E, NF = N / 2 + 1, M = N / 2;
+  static constexpr int PW = 32 / T;  // columns of a warp in the y passes
+  static constexpr int PADSH = E >= 16 ? 4 : 3;
+  // half a row, even so that pairs of FP32 columns stay 16-byte aligned
+  static constexpr int HP = ((N + (N >> PADSH)) / 2 > NF ? (N + (N >> PADSH)) / 2 : NF + 1) / 2 * 2;
+  static constexpr int RP = 2 * HP;
+  static constexpr int TWN = StageTw<P>::SIZE / 2 * 2 + 2;
+  static constexpr size_t SMEM = (size_t)(TWN + 3 * N * RP) * sizeof(cx<R>);
+  static constexpr int THREADS = N == 64 ? (sizeof(R) == 8 ? 512 : 256) : N == 32 ? 256 : 128;
+  static constexpr int MINB = N == 64 ? (sizeof(R) == 8 ? 1 : 2) : 1;
+  static constexpr int LINES = THREADS / T < N ? THREADS / T : N;  // z lines at a time
+  static_assert(T == 1 || LINES * T % 32 == 0, "a warp's lanes have all a line or need no barrier");
+  // n = 64: rows are a multiple of 128 bytes (FP64; 64 in FP32) apart, so the
+  // four columns of a warp's lanes change places from row to row
+  __device__ static __forceinline__ int sw(int row) {
+    if (N != 64) return 0;
+    return ((sizeof(R) == 8 ? row ^ (row >> 3) : (row >> 1) ^ (row >> 3)) & 1) << 2;
+  }
+};
+template <class R, int N>
+struct YZCol {  // position (row) of one column
+  int o;
+  __device__ __forceinline__ int operator()(int pos) const {
+    return pos * YZ<R, N>::RP + (o ^ YZ<R, N>::sw(pos));
+  }
+};
+template <class R, int N>
+struct YZRow {  // position in a pair's row
+  int s;
+  __device__ __forceinline__ int operator()(int pos) const {
+    return (pos + (pos >> YZ<R, N>::PADSH)) ^ s;
+  }
+};
+
+// extension of a pair of spectra to N positions, as in ext_gen
+template <class R, int N, class FAB>
+__device__ __forceinline__ void yz_ext(cx<R> (&y)[YZ<R, N>::E], int t, FAB fab) {
+  using C = cx<R>;
+  constexpr int M = N / 2;
+#pragma unroll
+  for (int e = 0; e < YZ<R, N>::E; e++) {
+    const int k = t + YZ<R, N>::T * e;
+    const bool direct = k <= M;
+    const int s = direct ? k : N - k;
+    C a, b;
+    fab(s, a, b);
+    if (s == 0 || s == M) {
+      a.y = 0;
+      b.y = 0;
+    }
+    if (!direct) {
+      a.y = -a.y;
+      b.y = -b.y;
+    }
+    y[e] = cmk<C>(a.x - b.y, a.y + b.x);
+  }
+}
+
+// grid: (n planes, nruns); KIND and KEEP as in the z pass
+template <class R, int N, int KIND, bool KEEP>
+__global__ void __launch_bounds__(YZ<R, N>::THREADS, YZ<R, N>::MINB)
+    k_yz(cx<R> *__restrict__ work, R *__restrict__ stale, const cx<R> *__restrict__ twg, Geo g,
+         R invn3, R *__restrict__ keep) {
+  using C = cx<R>;
+  using Y = YZ<R, N>;
+  using P = typename Y::P;
+  constexpr int E = Y::E, T = Y::T, RP = Y::RP, HP = Y::HP, NF = Y::NF, M = Y::M, PW = Y::PW;
+  constexpr int WARPS = Y::THREADS / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C *tw = (C *)smem_raw;
+  C *pl = tw + Y::TWN;
+  build_stage_tw<N, P>(tw, twg, N, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int plane = blockIdx.x;
+  work += (long long)blockIdx.y * g.run_spec + (long long)plane * N * g.nfp;
+  stale += (long long)blockIdx.y * g.run_real + (long long)plane * N * N;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+
+  {  // u, v, w, dv/dx and dw/dx to their places, all on their way at once
+    constexpr int V = 16 / (int)sizeof(C), CP = (NF + V - 1) / V;  // columns a copy, copies a row
+    for (int q = threadIdx.x; q < N * CP; q += Y::THREADS) {
+      const int row = q / CP, col = (q - row * CP) * V, o = row * g.nfp + col;
+      C *d = pl + row * RP;
+      const int a = col ^ Y::sw(row), b = (HP + col) ^ Y::sw(row);
+      copy16(d + a, work + SU * g.slot + o);
+      copy16(d + b, work + SDWDX * g.slot + o);
+      copy16(d + N * RP + a, work + SV * g.slot + o);
+      copy16(d + 2 * N * RP + a, work + SW * g.slot + o);
+      copy16(d + 2 * N * RP + b, work + SOMZ * g.slot + o);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
+
+  {  // y backward (B), in place
+    const int t = lane / PW, p = lane % PW;
+    constexpr int TILES = (NF + PW - 1) / PW;
+    for (int task = warp; task < 4 * TILES; task += WARPS) {
+      const int job = task / TILES;
+      // columns past the last repeat it (the same values to the same places)
+      const int c0 = (task % TILES) * PW + p, col = c0 < NF ? c0 : NF - 1;
+      const YZCol<R, N> lo{col}, hi{HP + col};
+      auto get = [&](C (&v)[E], const C *f, const YZCol<R, N> &idx) {
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = f[idx(t + T * e)];
+      };
+      auto fft = [&](C (&v)[E], C *f, const YZCol<R, N> &idx) {
+        if (T > 1) __syncwarp();  // the column has been read
+        line_fft<N, P, false>(v, t, tw, f, idx, WarpSync{});
+#pragma unroll
+        for (int e = 0; e < E; e++) f[idx(t + T * e)] = v[e];
+      };
+      C *f0 = pl, *f1 = pl + N * RP, *f2 = pl + 2 * N * RP;
+      C v[E];
+      if (job == 0) {  // omega_z = dv/dx - i ky u, and u
+        C u[E];
+        get(u, f0, lo);
+        get(v, f2, hi);
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+          const R k = (R)kwave(t + T * e, N);
+          v[e] = cmk<C>(fma_rn(k, u[e].y, v[e].x), fma_rn(-k, u[e].x, v[e].y));
+        }
+        fft(v, f2, hi);
+        fft(u, f0, lo);
+      } else if (job == 1) {  // dw/dy = i ky w, and w (not needed in the first stage)
+        C w[E];
+        get(w, f2, lo);
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+          const R k = (R)kwave(t + T * e, N);
+          v[e] = cmk<C>(mul_rn(-k, w[e].y), mul_rn(k, w[e].x));
+        }
+        fft(v, f1, hi);
+        if (KIND != 0) fft(w, f2, lo);
+      } else if (job == 2) {
+        get(v, f1, lo);
+        fft(v, f1, lo);
+      } else {
+        get(v, f0, hi);
+        fft(v, f0, hi);
+      }
+    }
+  }
+  __syncthreads();
+
+  const int KZ = g.kcut < M ? g.kcut : M;
+  for (int l0 = 0; l0 < N; l0 += Y::LINES) {  // z lines (C)
+    const int lid = threadIdx.x / T, t = threadIdx.x % T;
+    if (lid >= Y::LINES) break;  // whole warps, or T == 1
+    const int line = l0 + lid;
+    const YZRow<R, N> idx{Y::sw(line)};
+    C *r0 = pl + line * RP, *r1 = r0 + N * RP, *r2 = r1 + N * RP;
+    R *st = stale + line * N;
+    auto kp = [&](int f, int e, R v) {
+      if constexpr (KEEP)
+        keep[(6LL * blockIdx.y + f) * g.nreal + ((long long)plane * N + line) * N + t + T * e] = v;
+    };
+    auto at = [&](const C *r, int o) -> C { return r[o ^ idx.s]; };
+    auto fft_inv = [&](C (&y)[E], C *r) {
+      if (T > 1) __syncwarp();  // the row has been read
+      line_fft<N, P, false>(y, t, tw, r, idx, WarpSync{});
+    };
+    auto fft_fwd = [&](C (&y)[E], C *r) {
+      if (T > 1) __syncwarp();
+      line_fft<N, P, true>(y, t, tw, r, idx, WarpSync{});
+    };
+    auto f_ox = [&](int s) -> C {  // omega_x = dw/dy - i kz v
+      const C a = at(r1, HP + s), v = at(r1, s);
+      return cmk<C>(fma_rn((R)s, v.y, a.x), fma_rn(-(R)s, v.x, a.y));
+    };
+    auto f_oy = [&](int s) -> C {  // omega_y = i kz u - dw/dx
+      const C u = at(r0, s), d = at(r0, HP + s);
+      return cmk<C>(fma_rn(-(R)s, u.y, -d.x), fma_rn((R)s, u.x, -d.y));
+    };
+    auto out_z = [&](const C (&y)[E]) {  // N_z to the first half of pair 0
+#pragma unroll
+      for (int e = 0; e <= E / 2; e++) {
+        const int k = t + T * e;
+        if (k <= KZ) r0[k ^ idx.s] = y[e];
+      }
+    };
+    C y[E];
+    if constexpr (KIND == 0) {
+      R nx[E], ny[E];
+      auto sv = [&](int f, int e) -> R { return st[f * g.nreal + t + T * e]; };
+      yz_ext<R, N>(y, t, [&](int s, C &a, C &b) {
+        a = f_ox(s);
+        b = f_oy(s);
+      });
+      fft_inv(y, r0);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const R ox = y[e].x * invn3, oy = y[e].y * invn3;
+        const R u = sv(0, e), v = sv(1, e), w = sv(2, e);
+        nx[e] = mul_rn(-w, oy);
+        ny[e] = mul_rn(w, ox);
+        y[e] = cmk<C>(fma_rn(-v, ox, mul_rn(u, oy)), R(0));  // N_z
+        kp(3, e, ox);
+        kp(4, e, oy);
+      }
+      fft_fwd(y, r0);
+      out_z(y);
+      yz_ext<R, N>(y, t, [&](int s, C &a, C &b) {
+        a = at(r2, HP + s);
+        b = czero<C>();
+      });
+      fft_inv(y, r2);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const R oz = y[e].x * invn3;
+        y[e] = cmk<C>(fma_rn(sv(1, e), oz, nx[e]), fma_rn(-sv(0, e), oz, ny[e]));
+        kp(5, e, oz);
+      }
+    } else {
+      R su[E], soy[E], sv[E], sox[E];
+      yz_ext<R, N>(y, t, [&](int s, C &a, C &b) {
+        a = at(r0, s);
+        b = f_oy(s);
+      });
+      fft_inv(y, r0);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        su[e] = y[e].x * invn3;
+        soy[e] = y[e].y * invn3;
+        if (KIND == 2) st[t + T * e] = su[e];
+        kp(0, e, su[e]);
+        kp(4, e, soy[e]);
+      }
+      yz_ext<R, N>(y, t, [&](int s, C &a, C &b) {
+        a = at(r1, s);
+        b = f_ox(s);
+      });
+      fft_inv(y, r1);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const R v = y[e].x * invn3, ox = y[e].y * invn3;
+        sv[e] = v;
+        sox[e] = ox;
+        y[e] = cmk<C>(fma_rn(-v, ox, mul_rn(su[e], soy[e])), R(0));
+        if (KIND == 2) st[g.nreal + t + T * e] = v;
+        kp(1, e, v);
+        kp(3, e, ox);
+      }
+      fft_fwd(y, r1);
+      out_z(y);
+      yz_ext<R, N>(y, t, [&](int s, C &a, C &b) {
+        a = at(r2, s);
+        b = at(r2, HP + s);
+      });
+      fft_inv(y, r2);
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const R w = y[e].x * invn3, oz = y[e].y * invn3;
+        y[e] = cmk<C>(fma_rn(sv[e], oz, mul_rn(-w, soy[e])),
+                      fma_rn(w, sox[e], mul_rn(-su[e], oz)));
+        if (KIND == 2) st[2 * g.nreal + t + T * e] = w;
+        kp(2, e, w);
+        kp(5, e, oz);
+      }
+    }
+    fft_fwd(y, r2);
+#pragma unroll
+    for (int e = 0; e < E; e++) r2[idx(t + T * e)] = y[e];
+    if (T > 1) __syncwarp();
+#pragma unroll
+    for (int e = 0; e <= E / 2; e++) {  // N_x, N_y to pair 1
+      const int k = t + T * e;
+      if (k <= KZ) {
+        const C z = y[e], q = r2[idx((N - k) & (N - 1))];
+        const C a = cmk<C>(R(0.5) * (z.x + q.x), R(0.5) * (z.y - q.y));
+        const C d = cmk<C>(R(0.5) * (z.x - q.x), R(0.5) * (z.y + q.y));
+        r1[k ^ idx.s] = a;
+        r1[(HP + k) ^ idx.s] = cmk<C>(d.y, -d.x);  // -i d
+      }
+    }
+  }
+  __syncthreads();
+
+  {  // y forward (D), inside the 2/3 rule
+    const int t = lane / PW, p = lane % PW;
+    const int tiles = KZ / PW + 1;
+    for (int task = warp; task < 3 * tiles; task += WARPS) {
+      const int job = task / tiles;  // N_x, N_y, N_z
+      const int c0 = (task % tiles) * PW + p, col = c0 <= KZ ? c0 : KZ;
+      C *f = pl + (job == 2 ? 0 : N * RP);
+      const YZCol<R, N> idx{(job == 1 ? HP : 0) + col};
+      C v[E];
+#pragma unroll
+      for (int e = 0; e < E; e++) v[e] = f[idx(t + T * e)];
+      __syncwarp();
+      line_fft<N, P, true>(v, t, tw, f, idx, WarpSync{});
+      C *dst = work + (job == 0 ? SNX : job == 1 ? SNY : SNZ) * g.slot + col;
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const int k = kwave(t + T * e, N);
+        if ((k < 0 ? -k : k) <= g.kcut) dst[(t + T * e) * g.nfp] = v[e];
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -991,24 +1175,13 @@ struct XC {
   static constexpr int XB = (N + (N >> SH)) * W;  // exchange buffer
   static constexpr size_t SMEM = (size_t)(TWN + XB + 2 * N * W) * sizeof(cx<R>);
   static constexpr int WANT = (sizeof(R) == 8 ? 384 : 768) / THREADS;
-  static constexpr int MINB = WANT < 1 ? 1 : WANT > 16 ? 16 : WANT;  // blocks per SM
+  static constexpr int MINB = N <= 32 || WANT < 1 ? 1 : WANT;  // blocks per SM
 };
 template <int W, int SH>
 struct XIdx {
   int p;
   __device__ __forceinline__ int operator()(int pos) const { return (pos + (pos >> SH)) * W + p; }
 };
-
-// The x pass writes its roundings out (no product is left to be contracted
-// into a following addition at the compiler's choice): every kernel that
-// inlines it computes the same bits, and the value it stores is the one it
-// transforms on the spot.
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 
 // Outside the 2/3 rule dU = -c U_s with c = nu dt kk: the stage input that
 // stage ST forms (ST 3: the new state) is U_0 + m U_0 with this m.
@@ -1022,18 +1195,6 @@ __device__ __forceinline__ R lin_coef(R c) {
   const R m3 = mul_rn(-c, R(1) + m2);
   if (ST == 2) return m3;
   return fma_rn(m1 + R(2) * m2 + m3, R(1.0 / 3.0), mul_rn(mul_rn(-c, R(1) + m3), R(1.0 / 6.0)));
-}
-
-// loads that leave no line in L1 (little of it is left beside the buffers,
-// and lines reserved for loads in flight would bound how many there are)
-template <class C>
-__device__ __forceinline__ C ldcg(const C *p) {
-  return __ldcg(p);
-}
-// 16-byte asynchronous copy from global to shared memory, past L1
-__device__ __forceinline__ void copy16(void *dst, const void *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
 template <class R, int N, int ST, bool TAIL, class Sync>
@@ -1134,10 +1295,12 @@ __device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__re
     auto crow = [&](int ik) -> long long {
       return (long long)((unsigned)(ik < 0 ? ik + g.mk : ik) * crs);
     };
-    // state and stage inputs of a point, loaded a point ahead (as far as the
-    // compiler knows a store may alias a later load) except in stage 3, whose
-    // four triples leave no registers for it
-    constexpr bool AHEAD = ST < 3;
+    // State and stage inputs of a point: DEPTH points are on their way at a
+    // time (as far as the compiler knows a store may alias a later load).
+    // n <= 32, where latency is all, spends some 170 registers on them; else
+    // stage 3's four triples leave none for a second point.
+    constexpr int PER = 3 * (ST == 0 ? 1 : ST < 3 ? 2 : 4) * (int)sizeof(C) / 4;
+    constexpr int DEPTH = N <= 32 ? (170 / PER < E ? 170 / PER : E) : ST < 3 ? 2 : 1;
     struct In {
       C z[3], us[3], r1[3], r2[3];
     };
@@ -1155,6 +1318,12 @@ __device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__re
         }
       }
     };
+    In in[DEPTH];
+    auto load_first = [&]() {
+#pragma unroll
+      for (int e = 0; e + 1 < DEPTH; e++) load(in[e], e);
+    };
+    if (N <= 32) load_first();
     line_fft<N, P, true>(v, t, st, xb, idx, sync);
     copies_done();
 #pragma unroll
@@ -1170,8 +1339,7 @@ __device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__re
       s1[e * TH] = v[e];
       v[e] = y;
     }
-    In in0, in1;
-    if (AHEAD) load(in0, 0);
+    if (N > 32) load_first();
     line_fft<N, P, true>(v, t, st, xb, idx, sync);
     const R dtr = (R)dt, ky = (R)iky, kz = (R)col;
     auto update = [&](const In &q, int e) {
@@ -1227,10 +1395,8 @@ __device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__re
     };
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      In &cur = AHEAD && e % 2 ? in1 : in0, &nxt = AHEAD && e % 2 ? in0 : in1;
-      if (!AHEAD) load(cur, e);
-      if (AHEAD && e + 1 < E) load(nxt, e + 1);
-      update(cur, e);
+      if (e + DEPTH <= E) load(in[(e + DEPTH - 1) % DEPTH], e + DEPTH - 1);
+      update(in[e % DEPTH], e);
     }
   }
   if constexpr (!TAIL) return;

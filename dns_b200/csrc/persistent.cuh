@@ -76,7 +76,7 @@ struct PSync {
 // most PBS threads; the kernel holds the passes of each size it supports)
 __host__ __device__ constexpr bool p_supported_n(long n) { return n == 64 || n == 128; }
 
-// launch entry points, defined with the kernel in ens_persistent.cu (its own
+// launch entry points, defined with the kernel in ens_kernel.cuh (its own
 // translation unit: the kernel inlines every pass of every supported size)
 template <class R>
 cudaError_t p_prepare(size_t smem, int *blocks_per_sm);
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(PBS, PMinB<R>::value)
 // Self-test of the bounded wait: a barrier of one more block than the grid
 // has, which therefore never completes; the wait must give up after
 // wait_ns and report PERR_BARRIER_TIMEOUT.
-__global__ void k_barrier_selftest(PSync *sy, unsigned long long wait_ns) {
+static __global__ void k_barrier_selftest(PSync *sy, unsigned long long wait_ns) {
   grid_barrier(sy, gridDim.x + 1, wait_ns);
 }
 #endif  // DNSB_PERSISTENT_KERNELS

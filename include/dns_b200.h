@@ -167,8 +167,8 @@ int dns_synchronize(dns_ctx *ctx);
  * the kernels_per_step passes of a step into ms[] (stage-major order: stage 0
  * passes A x-inverse, B y-inverse, C z, D y-forward, E1 x-forward, E2 update,
  * stage 1 ..., stage 3).  A stage's E1 and E2 and the next stage's A are one
- * kernel, whose time is divided equally among them.  The state advances by
- * nsteps. */
+ * kernel, and for n <= 32 so are a stage's B, C and D; the time of such a
+ * kernel is divided equally among its passes.  The state advances by nsteps. */
 int dns_time_kernels(dns_ctx *ctx, double nu, double dt, long nsteps, double *ms);
 
 /* ---- ensemble: many independent runs stepped together ----
@@ -176,7 +176,8 @@ int dns_time_kernels(dns_ctx *ctx, double nu, double dt, long nsteps, double *ms
  * process-level ensembles (run.sh / hal.sh run one dns per core).  Runs of
  * any grid sizes and viscosities advance together, each following main.c's
  * step exactly (stale velocity included), under one of two schedules:
- *   batched     runs of equal n share batched kernel launches (16 per step),
+ *   batched     runs of equal n share batched kernel launches (16 per step, 8 for n <= 32
+ *               and three or more runs of 64),
  *               groups of different n run as concurrent branches of one
  *               CUDA graph launch per step;
  *   persistent  one cooperative kernel launch per step (captured in a CUDA
