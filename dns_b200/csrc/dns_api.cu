@@ -448,7 +448,8 @@ int set_coef(const Group &G, cudaStream_t st, const double *nu, const double *dt
 // reversed step; lambda of dU_s; two transform triples)
 enum { X_LA = 0, X_LB = 3, X_LDU = 6, X_T1 = 9, X_T2 = 12, NX = 15 };
 // real work triples (in units of n^3 fields)
-enum { RE_LN = 0, RE_LU = 3, RE_LOM = 6, RE_LSTALE = 9, NRE = 12 };
+// (lambda of N; of the velocity and of the vorticity; of the stale velocity)
+enum { RE_LN = 0, RE_LU = 3, RE_LSTALE = 9, NRE = 12 };
 
 struct Adj {
   Group G;
@@ -456,7 +457,7 @@ struct Adj {
   cudaGraphExec_t graph = nullptr, last = nullptr;  // dns_ctx's step and last
   char *arena = nullptr;
   void *sp = nullptr;        // [NX][slot], storage complex type
-  double *re = nullptr;      // [NRE][n^3] float64; LU, LOM hold the storage real type
+  double *re = nullptr;      // [NRE][n^3] float64; LU holds six fields of the storage real type
   char *snap_sp = nullptr;   // [S][3][slot]
   char *snap_re = nullptr;   // [S][3][n^3], storage real type
   char *keep = nullptr;      // [4][6][n^3], storage real type: the real velocity and
@@ -507,17 +508,21 @@ struct AdjOps {
     const unsigned cb = conv_blocks(g.nreal);
     // stage 0 reads the stale velocity (main.c:344), the step's input one
     const R *u = s > 0 ? A.K<R>(s, 0) : (const R *)G.stale;
-    k_adj_cross<R, R, R><<<cb, 256, 0, A.st>>>(u, A.K<R>(s, 3), A.Rf(RE_LN), lso, A.Rr<R>(RE_LU),
-                                               A.Rr<R>(RE_LOM), g.nreal);
-    O::r2c_fields(G, A.st, A.Rr<R>(RE_LOM), 3, A.X<C>(X_T1), t3);
-    if (s > 0) O::r2c_fields(G, A.st, A.Rr<R>(RE_LU), 3, A.X<C>(X_T2), t3);
+    R *lu = A.Rr<R>(RE_LU), *lom = lu + 3 * g.nreal;  // six fields side by side
+    k_adj_cross<R, R, R><<<cb, 256, 0, A.st>>>(u, A.K<R>(s, 3), A.Rf(RE_LN), lso, lu, lom, g.nreal);
+    // lambda of the velocity (not in stage 0) and of the vorticity in one batch
+    const int out[6] = {X_T2, X_T2 + 1, X_T2 + 2, X_T1, X_T1 + 1, X_T1 + 2};
+    if (s > 0)
+      O::r2c_fields(G, A.st, lu, 6, A.X<C>(0), out);
+    else
+      O::r2c_fields(G, A.st, lom, 3, A.X<C>(0), out + 3);
     k_adj_collect<256, C><<<pb, 256, 0, A.st>>>(
         A.X<C>(X_T1), s > 0 ? A.X<C>(X_T2) : nullptr, A.X<C>(X_LDU), Us, lin, lout, lacc, g, a,
         A.nu, A.dt, s > 0 ? RK_B[s - 1] : 0.0, s > 0 ? RK_A[s - 1] : 0.0, s > 0, A.part);
     k_dd_accumulate<256><<<1, 256, 0, A.st>>>(A.part, A.nblocks, A.acc_nu);
     if (s == 0)  // lambda of the step's input stale velocity, kept in float64
       k_real_convert<R, double><<<conv_blocks(3 * g.nreal), 256, 0, A.st>>>(
-          A.Rr<R>(RE_LU), A.Rf(RE_LSTALE), 3 * g.nreal);
+          lu, A.Rf(RE_LSTALE), 3 * g.nreal);
     CKL();
     return DNS_OK;
   }
