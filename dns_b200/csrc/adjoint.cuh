@@ -102,29 +102,137 @@ __global__ void k_adj_lamN(const C *__restrict__ ldU, C *__restrict__ out, Geo g
   }
 }
 
-// lu = om x lN (+ lstale_out), lom = lN x u   on [3][n^3] real arrays (u,
-// om and the outputs in the precision they are kept in, the rest float64)
-template <class RU, class RW, class RO>
-__global__ void k_adj_cross(const RU *__restrict__ u, const RW *__restrict__ om,
-                            const double *__restrict__ lN, const double *__restrict__ lstale_out,
-                            RO *__restrict__ lu, RO *__restrict__ lom, long long nr) {
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nr;
-       q += (long long)gridDim.x * blockDim.x) {
-    const double ux = u[q], uy = u[nr + q], uz = u[2 * nr + q];
-    const double wx = om[q], wy = om[nr + q], wz = om[2 * nr + q];
-    const double lx = lN[q], ly = lN[nr + q], lz = lN[2 * nr + q];
-    double ax = wy * lz - wz * ly, ay = wz * lx - wx * lz, az = wx * ly - wy * lx;
-    if (lstale_out) {
-      ax += lstale_out[q];
-      ay += lstale_out[nr + q];
-      az += lstale_out[2 * nr + q];
+// The z part of a transposed stage, per z line: lambda_N (slots 0-2 of work,
+// zero past kcut) to real space, with the stage's real velocity u and
+// vorticity om
+//   lambda_u = om x lambda_N (+ lst),  lambda_om = lambda_N x u
+// in FP64, rounded once to the storage type, and their forward transforms:
+// lambda_om to slots 0-2, lambda_u to slots 3-5, or with LAST (stage 0, whose
+// velocity is the stale one) lambda_u itself, real, to lst_out.  Two real
+// transforms run as one complex one, as in the z pass.  One kernel in place
+// of a c2r, a pointwise and two r2c passes: 15 slots of traffic a stage, not
+// 33.
+template <class R, int N>
+struct ZA {
+  using P = Plan<N>;
+  static constexpr int E = P::E, T = N / E, M = N / 2;
+  static constexpr int THREADS = (N * N * T) < 128 ? (N * N * T) : 128;
+  static constexpr int LINES = THREADS / T;
+  static constexpr int PADSH = E >= 16 ? 4 : 3;
+  static constexpr int XB = N + (N >> PADSH);
+  static constexpr int TWN = StageTw<P>::SIZE / 2 * 2 + 2;
+  static constexpr size_t SMEM = (size_t)(TWN + LINES * XB) * sizeof(cx<R>) + (size_t)LINES * 3 * N * sizeof(R);
+  static constexpr int MINB = sizeof(R) == 8 ? 2 : 4;
+};
+template <class R, int N, bool LAST>
+__global__ void __launch_bounds__(ZA<R, N>::THREADS, ZA<R, N>::MINB)
+    k_zadj(cx<R> *work, const R *__restrict__ u, const R *__restrict__ om,
+           const double *__restrict__ lst, double *__restrict__ lst_out,
+           const cx<R> *__restrict__ twg, Geo g) {
+  using C = cx<R>;
+  using Z = ZA<R, N>;
+  constexpr int E = Z::E, T = Z::T, M = Z::M;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C *tw = (C *)smem_raw;
+  build_stage_tw<N, typename Z::P>(tw, twg, N, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const int lid = threadIdx.x / T, t = threadIdx.x % T;
+  C *xb = tw + Z::TWN + lid * Z::XB;
+  R *sl = (R *)(tw + Z::TWN + Z::LINES * Z::XB) + lid * 3 * N + t;  // own points: sl[f * N + T * e]
+  const long long line = (long long)blockIdx.x * Z::LINES + lid;  // N * N is a multiple of LINES
+  C *row = work + line * g.nfp;
+  const long long r0 = line * N + t;
+  const LineSync<(T > 32)> sync{};
+  const PadShift<Z::PADSH> idx{};
+  C y[E];
+  auto ext = [&](const C *a, const C *b) {  // the pair's Hermitian extension
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const int k = t + T * e;
+      const bool direct = k <= M;
+      const int q = direct ? k : N - k;
+      C va = q <= g.kcut ? a[q] : czero<C>();
+      C vb = b && q <= g.kcut ? b[q] : czero<C>();
+      if (q == 0 || q == M) {
+        va.y = 0;
+        vb.y = 0;
+      }
+      if (!direct) {
+        va.y = -va.y;
+        vb.y = -vb.y;
+      }
+      y[e] = cmk<C>(va.x - vb.y, va.y + vb.x);
     }
-    lu[q] = (RO)ax;
-    lu[nr + q] = (RO)ay;
-    lu[2 * nr + q] = (RO)az;
-    lom[q] = (RO)(ly * uz - lz * uy);
-    lom[nr + q] = (RO)(lz * ux - lx * uz);
-    lom[2 * nr + q] = (RO)(lx * uy - ly * ux);
+  };
+  ext(row, row + g.slot);
+  line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    sl[T * e] = y[e].x;
+    sl[N + T * e] = y[e].y;
+  }
+  ext(row + 2 * g.slot, nullptr);
+  line_fft<N, typename Z::P, false>(y, t, tw, xb, idx, sync);
+#pragma unroll
+  for (int e = 0; e < E; e++) sl[2 * N + T * e] = y[e].x;
+
+  // component f of the cross product of two fields at own point e: from lambda_N
+  // and the velocity (OM) or from the vorticity and lambda_N
+  auto l_ = [&](int f, int e) -> double { return sl[f * N + T * e]; };
+  auto lom = [&](int f, int e) -> R {
+    const int a = (f + 1) % 3, b = (f + 2) % 3;
+    const double ua = u[a * g.nreal + r0 + T * e], ub = u[b * g.nreal + r0 + T * e];
+    return (R)(l_(a, e) * ub - l_(b, e) * ua);
+  };
+  auto lu = [&](int f, int e) -> R {
+    const int a = (f + 1) % 3, b = (f + 2) % 3;
+    const double wa = om[a * g.nreal + r0 + T * e], wb = om[b * g.nreal + r0 + T * e];
+    double v = wa * l_(b, e) - wb * l_(a, e);
+    if (lst) v += lst[f * g.nreal + r0 + T * e];
+    return (R)v;
+  };
+  // forward transform of the pair in y into two slots (the second may be none)
+  auto out = [&](int sa, int sb) {
+    line_fft<N, typename Z::P, true>(y, t, tw, xb, idx, sync);
+    C *oa = row + sa * g.slot, *ob = row + sb * g.slot;
+    if (sb < 0) {
+#pragma unroll
+      for (int e = 0; e <= E / 2; e++)
+        if (t + T * e <= M) oa[t + T * e] = y[e];
+      return;
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++) xb[idx(t + T * e)] = y[e];
+    sync();
+#pragma unroll
+    for (int e = 0; e <= E / 2; e++) {
+      const int k = t + T * e;
+      if (k <= M) {
+        const C z = y[e], p = xb[idx((N - k) & (N - 1))];
+        oa[k] = cmk<C>(R(0.5) * (z.x + p.x), R(0.5) * (z.y - p.y));
+        ob[k] = cmk<C>(R(0.5) * (z.y + p.y), -R(0.5) * (z.x - p.x));  // -i (Z - conj P) / 2
+      }
+    }
+    sync();
+  };
+#pragma unroll
+  for (int e = 0; e < E; e++) y[e] = cmk<C>(lom(0, e), lom(1, e));
+  out(0, 1);
+  if constexpr (LAST) {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      y[e] = cmk<C>(lom(2, e), R(0));
+#pragma unroll
+      for (int f = 0; f < 3; f++) lst_out[f * g.nreal + r0 + T * e] = (double)lu(f, e);
+    }
+    out(2, -1);
+  } else {
+#pragma unroll
+    for (int e = 0; e < E; e++) y[e] = cmk<C>(lom(2, e), lu(0, e));
+    out(2, 3);
+#pragma unroll
+    for (int e = 0; e < E; e++) y[e] = cmk<C>(lu(1, e), lu(2, e));
+    out(4, 5);
   }
 }
 

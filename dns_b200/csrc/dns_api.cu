@@ -448,8 +448,8 @@ int set_coef(const Group &G, cudaStream_t st, const double *nu, const double *dt
 // reversed step; lambda of dU_s; two transform triples)
 enum { X_LA = 0, X_LB = 3, X_LDU = 6, X_T1 = 9, X_T2 = 12, NX = 15 };
 // real work triples (in units of n^3 fields)
-// (lambda of N; of the velocity and of the vorticity; of the stale velocity)
-enum { RE_LN = 0, RE_LU = 3, RE_LSTALE = 9, NRE = 12 };
+// (the gradient as it leaves; lambda of the stale velocity)
+enum { RE_OUT = 0, RE_LSTALE = 3, NRE = 6 };
 
 struct Adj {
   Group G;
@@ -457,7 +457,7 @@ struct Adj {
   cudaGraphExec_t graph = nullptr, last = nullptr;  // dns_ctx's step and last
   char *arena = nullptr;
   void *sp = nullptr;        // [NX][slot], storage complex type
-  double *re = nullptr;      // [NRE][n^3] float64; LU holds six fields of the storage real type
+  double *re = nullptr;      // [NRE][n^3] float64
   char *snap_sp = nullptr;   // [S][3][slot]
   char *snap_re = nullptr;   // [S][3][n^3], storage real type
   char *keep = nullptr;      // [4][6][n^3], storage real type: the real velocity and
@@ -469,9 +469,6 @@ struct Adj {
   template <class C>
   C *X(int i) const { return (C *)sp + (size_t)i * G.g.slot; }
   double *Rf(int i) const { return re + (size_t)i * G.g.nreal; }
-  // a real triple seen in the storage type (3 n^3 values fit in its space)
-  template <class R>
-  R *Rr(int i) const { return (R *)(re + (size_t)i * G.g.nreal); }
   size_t slot3() const { return (size_t)3 * G.g.slot * G.csize; }
   size_t real3() const { return (size_t)3 * G.g.nreal * G.rsize; }
   size_t real3d() const { return (size_t)3 * G.g.nreal * sizeof(double); }
@@ -483,6 +480,10 @@ template <class R, int N>
 struct AdjOps {
   using O = Ops<R, N>;
   using C = cx<R>;
+  static cudaError_t setup() {
+    const cudaError_t e = O::allow(k_zadj<R, N, false>, ZA<R, N>::SMEM);
+    return e == cudaSuccess ? O::allow(k_zadj<R, N, true>, ZA<R, N>::SMEM) : e;
+  }
   static unsigned pblocks(const Adj &A) { return (unsigned)A.nblocks; }
 
   // U_s: the step input (slot SA, untouched by the forward stages 0-2) and
@@ -503,26 +504,31 @@ struct AdjOps {
     const StageIn<C> Us = stage_input(A, s);
     const unsigned pb = pblocks(A);
     k_adj_lamN<C><<<pb, 256, 0, A.st>>>(A.X<C>(X_LDU), A.X<C>(X_T1), g, A.dt);
-    O::c2r_fields(G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_LN), 1.0);
-    const double *lso = s == 3 ? A.Rf(RE_LSTALE) : nullptr;
-    const unsigned cb = conv_blocks(g.nreal);
+    // lambda of N along x and y, the z part, and lambda of the vorticity and
+    // (not in stage 0) of the velocity along y and x, as one batch
+    C *wk = O::slot(G, SLOT_WORK);
+    ColJobs jx = jobs_map(t3, t3, 3), jy = jx;
+    O::template colpass_io<0, false>(G, A.st, A.X<C>(X_T1), wk, jx, 1);
+    O::template colpass_io<1, false>(G, A.st, wk, wk, jy, 1);
     // stage 0 reads the stale velocity (main.c:344), the step's input one
     const R *u = s > 0 ? A.K<R>(s, 0) : (const R *)G.stale;
-    R *lu = A.Rr<R>(RE_LU), *lom = lu + 3 * g.nreal;  // six fields side by side
-    k_adj_cross<R, R, R><<<cb, 256, 0, A.st>>>(u, A.K<R>(s, 3), A.Rf(RE_LN), lso, lu, lom, g.nreal);
-    // lambda of the velocity (not in stage 0) and of the vorticity in one batch
-    const int out[6] = {X_T2, X_T2 + 1, X_T2 + 2, X_T1, X_T1 + 1, X_T1 + 2};
+    const dim3 grid(N * N / ZA<R, N>::LINES);
     if (s > 0)
-      O::r2c_fields(G, A.st, lu, 6, A.X<C>(0), out);
+      k_zadj<R, N, false><<<grid, ZA<R, N>::THREADS, ZA<R, N>::SMEM, A.st>>>(
+          wk, u, A.K<R>(s, 3), s == 3 ? A.Rf(RE_LSTALE) : nullptr, nullptr, O::tw(G), g);
     else
-      O::r2c_fields(G, A.st, lom, 3, A.X<C>(0), out + 3);
+      k_zadj<R, N, true><<<grid, ZA<R, N>::THREADS, ZA<R, N>::SMEM, A.st>>>(
+          wk, u, A.K<R>(s, 3), nullptr, A.Rf(RE_LSTALE), O::tw(G), g);
+    const int in[6] = {0, 1, 2, 3, 4, 5};
+    const int to[6] = {X_T1, X_T1 + 1, X_T1 + 2, X_T2, X_T2 + 1, X_T2 + 2};
+    jy = jobs_map(in, in, s > 0 ? 6 : 3);
+    jx = jobs_map(in, to, s > 0 ? 6 : 3);
+    O::template colpass_io<1, true>(G, A.st, wk, wk, jy, 1);
+    O::template colpass_io<0, true>(G, A.st, wk, A.X<C>(0), jx, 1);
     k_adj_collect<256, C><<<pb, 256, 0, A.st>>>(
         A.X<C>(X_T1), s > 0 ? A.X<C>(X_T2) : nullptr, A.X<C>(X_LDU), Us, lin, lout, lacc, g, a,
         A.nu, A.dt, s > 0 ? RK_B[s - 1] : 0.0, s > 0 ? RK_A[s - 1] : 0.0, s > 0, A.part);
     k_dd_accumulate<256><<<1, 256, 0, A.st>>>(A.part, A.nblocks, A.acc_nu);
-    if (s == 0)  // lambda of the step's input stale velocity, kept in float64
-      k_real_convert<R, double><<<conv_blocks(3 * g.nreal), 256, 0, A.st>>>(
-          lu, A.Rf(RE_LSTALE), 3 * g.nreal);
     CKL();
     return DNS_OK;
   }
@@ -1403,6 +1409,14 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
       if (e != cudaSuccess) r = fail(DNS_ERR_CUDA, cudaGetErrorString(e), __FILE__, __LINE__);
     }
   }
+  if (r == DNS_OK) {
+    cudaError_t e = cudaSuccess;
+    dispatch(A.G, [&](auto ops) {
+      using O = decltype(ops);
+      e = AdjOps<typename O::Real, O::Nval>::setup();
+    });
+    if (e != cudaSuccess) r = fail(DNS_ERR_CUDA, cudaGetErrorString(e), __FILE__, __LINE__);
+  }
   if (r == DNS_OK) r = group_build_graph(A.G, A.st, true, &A.graph);
   if (r == DNS_OK) r = group_build_graph(A.G, A.st, false, &A.last);
   // J alone: the forward sweep is all it takes (no snapshots are needed
@@ -1451,14 +1465,14 @@ int dns_adjoint_energy_prec(long n, int precision, const double *U, const double
       using O = decltype(ops);
       using C = typename O::C;
       k_div_wz3<C><<<A.nblocks, 256, 0, A.st>>>(A.X<C>(A.lhat), A.X<C>(X_T1), g);
-      O::c2r_fields(A.G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_LN), 1.0);
+      O::c2r_fields(A.G, A.st, A.X<C>(X_T1), t3, 3, A.Rf(RE_OUT), 1.0);
     });
-    k_add_real<<<conv_blocks(3 * g.nreal), 256, 0, A.st>>>(A.Rf(RE_LSTALE), A.Rf(RE_LN), 3 * g.nreal);
+    k_add_real<<<conv_blocks(3 * g.nreal), 256, 0, A.st>>>(A.Rf(RE_LSTALE), A.Rf(RE_OUT), 3 * g.nreal);
     cudaError_t e = cudaGetLastError();
     double *dst[3] = {gU, gV, gW};
     for (int f = 0; f < 3 && e == cudaSuccess; f++)
       if (dst[f])
-        e = cudaMemcpyAsync(dst[f], A.Rf(RE_LN + f), (size_t)g.nreal * sizeof(double),
+        e = cudaMemcpyAsync(dst[f], A.Rf(RE_OUT + f), (size_t)g.nreal * sizeof(double),
                             cudaMemcpyDeviceToHost, A.st);
     double4 gn = make_double4(0, 0, 0, 0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&gn, A.acc_nu, sizeof(double4), cudaMemcpyDeviceToHost, A.st);

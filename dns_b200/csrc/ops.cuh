@@ -547,21 +547,6 @@ struct Ops {
     colpass_io<1, false>(G, st, wk, wk, j2, 1);
     k_zc2r<R, N><<<zgrid(K), ZCfg<N>::THREADS, Z_SMEM, st>>>(wk, out, tw(G), G.g, scale);
   }
-  // r2c of K real fields in[f * nreal] into spectral out + out_slots[f] * slot
-  static void r2c_fields(const Group &G, cudaStream_t st, const R *in, int K, C *out,
-                         const int *out_slots) {
-    C *wk = slot(G, SLOT_WORK);
-    ColJobs j1 = jobs_empty(K), j2 = jobs_empty(K);
-    for (int f = 0; f < K; f++) {
-      j1.in_slot[f] = f;
-      j1.out_slot[f] = out_slots[f];
-      j2.in_slot[f] = f;
-      j2.out_slot[f] = f;
-    }
-    k_zr2c<R, N><<<zgrid(K), ZCfg<N>::THREADS, Z_SMEM, st>>>(in, wk, tw(G), G.g);
-    colpass_io<1, true>(G, st, wk, wk, j2, 1);
-    colpass_io<0, true>(G, st, wk, out, j1, 1);
-  }
 
   // energy / enstrophy sums of every run into diag_out[run]
   static void diag(const Group &G, cudaStream_t st) {
