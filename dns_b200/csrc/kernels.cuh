@@ -1265,17 +1265,6 @@ __device__ __forceinline__ void xstage_body(const XArgs<R> &a, const cx<R> *__re
     if (sizeof(C) != 16) __syncwarp();
   };
   auto landed = [&](const C *s, int e) { return first_ok ? s[e * TH] : czero<C>(); };
-  // n = 512: one block has the SM to itself, and nothing else hides the waits
-  // on the state's rows in the update: they are brought to L2 meanwhile (middle
-  // stage FP64 3.56 -> 3.47 ms, FP32 1.86 -> 1.79; at n = 256, with three blocks
-  // an SM, 0.359 -> 0.365)
-  if (N == 512 && hasn) {
-#pragma unroll
-    for (int e = p; e < E; e += W)
-#pragma unroll
-      for (int f = 0; f < 3; f++)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(u0 - p + at(e) + f * g.slot));
-  }
   build_stage_tw<N, P>(st, twg, N, b.tid, b.nt);
   sync();
 
