@@ -905,7 +905,7 @@ __global__ void __launch_bounds__(YZ<R, N>::THREADS, YZ<R, N>::MINB)
         for (int e = 0; e < E; e++) v[e] = f[idx(t + T * e)];
       };
       auto fft = [&](C (&v)[E], C *f, const YZCol<R, N> &idx) {
-        if (T > 1) __syncwarp();  // the column has been read
+        __syncwarp();  // the column has been read, also by the lanes that repeat it
         line_fft<N, P, false>(v, t, tw, f, idx, WarpSync{});
 #pragma unroll
         for (int e = 0; e < E; e++) f[idx(t + T * e)] = v[e];
