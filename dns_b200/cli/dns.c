@@ -285,8 +285,8 @@ int main(int argc, char **argv) {
   }
   /* Opt-in kernel timings (no counterpart in the reference):
    * DNS_B200_TIMINGS=<k> times k more steps launch by launch after the run
-   * (the printed history is complete before) and prints each kernel's mean
-   * time to stderr. */
+   * (the printed history is complete before) and prints each pass's mean time
+   * to stderr, that of a pass which shares a kernel as its third of it. */
   const char *tenv = getenv("DNS_B200_TIMINGS");
   if (tenv && atol(tenv) > 0) {
     static const char *pass[6] = {"A x-inverse", "B y-inverse", "C z-fused",
@@ -303,7 +303,12 @@ int main(int argc, char **argv) {
       die_status("dns_time_kernels", st);
     double sum = 0.0;
     for (int q = 0; q < info.kernels_per_step; q++) {
-      fprintf(stderr, "dns: stage %d %s: %.4f ms\n", q / 6, pass[q % 6], ms[q]);
+      const int p = q % 6;
+      const char *share = p == 0 || p >= 4 ? " (a third of the kernel of E1, E2 and the next A)"
+                          : info.n <= 32   ? " (a third of the kernel of B, C and D)"
+                                           : "";
+      /* no ": " may follow the time: programs split the line there */
+      fprintf(stderr, "dns: stage %d %s: %.4f ms%s\n", q / 6, pass[p], ms[q], share);
       sum += ms[q];
     }
     fprintf(stderr, "dns: step (sum of its kernels): %.4f ms over %ld steps\n", sum, atol(tenv));

@@ -911,20 +911,20 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
     c->cur_nu = nu;
     c->cur_dt = dt;
   }
-  // the launches of a step: the x transform of the state, then each stage's
-  // kernels, with the passes each of them runs (the x pass a stage's E1 and
-  // E2 and, except in the last, the next one's A)
+  // the launches of a step in the middle of a dns_step call, with the passes
+  // each of them runs: the x pass a stage's E1 and E2 and the next stage's A,
+  // the last stage's that of the next step
   const int K = c->kernels_per_step;
   struct Launch {
-    int s, k, first, count;
+    int s, k, first, count;  // passes first, first + 1, ..., modulo K
   };
-  std::vector<Launch> launches{{-1, K_X, 0, 1}};
+  std::vector<Launch> launches;
   dispatch(c->grp, [&](auto ops) {
     using O = decltype(ops);
     for (int s = 0; s < 4; s++)
       for (int q = 0; q < O::kernels(c->grp); q++) {
         const int k = O::kernel(c->grp, q), p0 = s * PASSES_PER_STAGE;
-        launches.push_back(k == K_X    ? Launch{s, k, p0 + 4, s < 3 ? 3 : 2}
+        launches.push_back(k == K_X    ? Launch{s, k, p0 + 4, 3}
                            : k == K_YZ ? Launch{s, k, p0 + 1, 3}
                                        : Launch{s, k, p0 + 1 + k, 1});
       }
@@ -942,12 +942,13 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
   std::vector<cudaEvent_t> &ev = evs.v;
   for (auto &e : ev) CK(cudaEventCreate(&e));
   for (int k = 0; k < K; k++) ms[k] = 0.0;
-  int st = DNS_OK;
+  dispatch(c->grp, [&](auto ops) { decltype(ops)::first(c->grp, c->stream); });
+  int st = check_launch(__FILE__, __LINE__);
   for (long s = 0; s < nsteps && st == DNS_OK; s++) {
     CK(cudaEventRecord(ev[0], c->stream));
     for (int k = 0; k < L; k++) {
       dispatch(c->grp, [&](auto ops) {
-        decltype(ops)::stage_kernel(c->grp, c->stream, launches[k].s, launches[k].k, false);
+        decltype(ops)::stage_kernel(c->grp, c->stream, launches[k].s, launches[k].k, true);
       });
       CK(cudaEventRecord(ev[k + 1], c->stream));
     }
@@ -956,7 +957,8 @@ int dns_time_kernels(dns_ctx *c, double nu, double dt, long nsteps, double *ms) 
     for (int k = 0; k < L; k++) {
       float t = 0.f;
       CK(cudaEventElapsedTime(&t, ev[k], ev[k + 1]));
-      for (int p = 0; p < launches[k].count; p++) ms[launches[k].first + p] += t / launches[k].count;
+      for (int p = 0; p < launches[k].count; p++)
+        ms[(launches[k].first + p) % K] += t / launches[k].count;
     }
   }
   for (int k = 0; k < K; k++) ms[k] /= (double)nsteps;

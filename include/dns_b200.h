@@ -137,8 +137,9 @@ typedef struct {
   unsigned flags;
   size_t device_bytes;     /* device memory held by the context */
   size_t slot_bytes;       /* bytes of one padded spectral field */
-  int kernels_per_step;    /* passes of one RK4 step, the entries that
-                              dns_time_kernels writes */
+  int kernels_per_step;    /* passes of one RK4 step (24), the entries that
+                              dns_time_kernels writes; they run as 16
+                              launches, for n <= 32 as 8 */
 } dns_info_t;
 int dns_get_info(dns_ctx *ctx, dns_info_t *info);
 /* The kernel schedule the library's autotuner chose for this context's grid
@@ -162,13 +163,15 @@ void *dns_get_stream(dns_ctx *ctx);
 /* Wait for all work queued on the context's stream. */
 int dns_synchronize(dns_ctx *ctx);
 
-/* Time each pass of the step: runs nsteps steps launch by launch with CUDA
- * events between kernels and writes the mean time in milliseconds of each of
+/* Time each pass of the step: runs nsteps steps, in the form that dns_step
+ * repeats in the middle of a call, launch by launch with CUDA events between
+ * kernels (the x transform that opens a call is not timed) and writes the mean time in milliseconds of each of
  * the kernels_per_step passes of a step into ms[] (stage-major order: stage 0
  * passes A x-inverse, B y-inverse, C z, D y-forward, E1 x-forward, E2 update,
- * stage 1 ..., stage 3).  A stage's E1 and E2 and the next stage's A are one
- * kernel, and for n <= 32 so are a stage's B, C and D; the time of such a
- * kernel is divided equally among its passes.  The state advances by nsteps. */
+ * stage 1 ..., stage 3).  A stage's E1 and E2 and the next stage's A (stage
+ * 3's: the next step's) are one kernel, and for n <= 32 so are a stage's B, C
+ * and D; each pass of such a kernel is given a third of its time, whatever it
+ * takes of it.  The state advances by nsteps. */
 int dns_time_kernels(dns_ctx *ctx, double nu, double dt, long nsteps, double *ms);
 
 /* ---- ensemble: many independent runs stepped together ----
