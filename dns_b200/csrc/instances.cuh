@@ -11,9 +11,7 @@ namespace dnsb {
 #define DNSB_COL(R, N, A, F)                                                             \
   extern template __global__ void k_colpass<R, N, A, F>(                                 \
       const cx<R> *__restrict__, cx<R> *__restrict__, const cx<R> *__restrict__, Geo, ColJobs); \
-  DNSB_COL_M(R, N, A, F, 1) DNSB_COL_M(R, N, A, F, 2) DNSB_COL_M(R, N, A, F, 3)          \
-  DNSB_COL_M(R, N, A, F, 4) DNSB_COL_M(R, N, A, F, 5) DNSB_COL_M(R, N, A, F, 6)          \
-  DNSB_COL_M(R, N, A, F, 8) DNSB_COL_M(R, N, A, F, 10) DNSB_COL_M(R, N, A, F, 12)
+  DNSB_COL_MINB(DNSB_COL_M, R, N, A, F)
 #define DNSB_X(R, N, S, T) \
   extern template __global__ void k_xstage<R, N, S, T>(XArgs<R>, const cx<R> *__restrict__, Geo);
 #define DNSB_SIZE(R, N)                                                                  \
@@ -30,8 +28,8 @@ namespace dnsb {
                                                       const cx<R> *__restrict__, Geo, R, \
                                                       R *__restrict__);
 #define DNSB_PLANE(R, N)                                                                 \
-  DNSB_YZ(R, N, 0, false) DNSB_YZ(R, N, 1, false) DNSB_YZ(R, N, 2, false) \
-  DNSB_YZ(R, N, 0, true) DNSB_YZ(R, N, 1, true)
+  DNSB_YZ(R, N, 0, false) DNSB_YZ(R, N, 1, false) DNSB_YZ(R, N, 2, false)
+#define DNSB_PLANE_KEEP(R, N) DNSB_YZ(R, N, 0, true) DNSB_YZ(R, N, 1, true)
 #define DNSB_Z(R, N, K)                                                                  \
   extern template __global__ void k_zstage<R, N, K>(cx<R> *__restrict__, R *__restrict__, \
                                                     const cx<R> *__restrict__, Geo, R);
@@ -43,6 +41,7 @@ namespace dnsb {
   DNSB_Z(R, N, 0) DNSB_Z(R, N, 1) DNSB_Z(R, N, 2) DNSB_ZK(R, N, 0) DNSB_ZK(R, N, 1)
 #define DNSB_PRECISION(R)                                                                \
   DNSB_PLANE(R, 8) DNSB_PLANE(R, 16) DNSB_PLANE(R, 32) DNSB_PLANE(R, 64)                 \
+  DNSB_PLANE_KEEP(R, 8) DNSB_PLANE_KEEP(R, 16) DNSB_PLANE_KEEP(R, 32)                    \
   DNSB_LINES(R, 64) DNSB_LINES(R, 128) DNSB_LINES(R, 256) DNSB_LINES(R, 512)             \
   DNSB_SIZE(R, 8) DNSB_SIZE(R, 16) DNSB_SIZE(R, 32) DNSB_SIZE(R, 64)                     \
   DNSB_SIZE(R, 128) DNSB_SIZE(R, 256) DNSB_SIZE(R, 512)

@@ -80,7 +80,7 @@ struct Geo {
 // pass (the y forward pass of N, whose result only enters the update inside
 // the 2/3 rule, main.c:381-386) is launched on the column tiles that hold
 // kz <= kcut only and stores only |ky| <= kcut.
-struct ColJobs {
+struct ColJobs {  // der_slot and add_slot: y only
   int in_slot[8];
   int out_slot[8];   // -1: no plain output
   int der_slot[8];   // -1: no derivative output
@@ -183,7 +183,9 @@ __device__ __forceinline__ void colpass_body(const cx<R> *__restrict__ in, cx<R>
     rs = g.nfp;
   }
   const C *src = in + (long long)jobs.in_slot[job] * g.slot + base;
-  const int oslot = jobs.out_slot[job], dslot = jobs.der_slot[job], aslot = jobs.add_slot[job];
+  // derivatives are taken along y only (the x pass of a step forms its own)
+  const int oslot = jobs.out_slot[job], dslot = AXIS == 1 ? jobs.der_slot[job] : -1,
+            aslot = jobs.add_slot[job];
   C v[E];
   // the input is read twice (the second read is an L2 hit) rather than kept
   // in a second register array: first for the derivative i k f, then for the
@@ -244,6 +246,16 @@ __global__ void __launch_bounds__((N / Plan<N>::E) * ColW<R, AXIS, N>::W, MINB)
 // (0: the compiler's register choice; otherwise register caps of about 170,
 // 128, 102, 85, 64; FP64 tiles stop at 80: at 64 they spill a kilobyte per
 // thread).
+// DNSB_COL_MINB lists every m > 0, for the declarations of instances.cuh: a
+// candidate missing from it would be compiled again in each unit that uses it.
+#define DNSB_COL_MINB(X, ...)                                                        \
+  X(__VA_ARGS__, 1) X(__VA_ARGS__, 2) X(__VA_ARGS__, 3) X(__VA_ARGS__, 4) X(__VA_ARGS__, 5) \
+  X(__VA_ARGS__, 6) X(__VA_ARGS__, 8) X(__VA_ARGS__, 10) X(__VA_ARGS__, 12)
+constexpr bool col_minb_listed(int m) {
+#define DNSB_COL_IS(M, V) || M == V
+  return false DNSB_COL_MINB(DNSB_COL_IS, m);
+#undef DNSB_COL_IS
+}
 template <int THREADS, int CB>
 struct ColCands {
   static constexpr int n = 1;
@@ -856,7 +868,8 @@ __device__ __forceinline__ void yz_ext(cx<R> (&y)[YZ<R, N>::E], int t, FAB fab) 
   }
 }
 
-// grid: (n planes, nruns); KIND and KEEP as in the z pass
+// grid: (n planes, nruns); KIND and KEEP as in the z pass (KEEP: one run, so
+// n <= 32, where one run takes this kernel)
 template <class R, int N, int KIND, bool KEEP>
 __global__ void __launch_bounds__(YZ<R, N>::THREADS, YZ<R, N>::MINB)
     k_yz(cx<R> *__restrict__ work, R *__restrict__ stale, const cx<R> *__restrict__ twg, Geo g,
@@ -954,7 +967,7 @@ __global__ void __launch_bounds__(YZ<R, N>::THREADS, YZ<R, N>::MINB)
     R *st = stale + line * N;
     auto kp = [&](int f, int e, R v) {
       if constexpr (KEEP)
-        keep[(6LL * blockIdx.y + f) * g.nreal + ((long long)plane * N + line) * N + t + T * e] = v;
+        keep[f * g.nreal + ((long long)plane * N + line) * N + t + T * e] = v;
     };
     auto at = [&](const C *r, int o) -> C { return r[o ^ idx.s]; };
     auto fft_inv = [&](C (&y)[E], C *r) {

@@ -140,6 +140,7 @@ struct Ops {
   template <int AXIS, bool FWD, int I>
   static ColFn col_cand() {
     constexpr int m = Cands<AXIS>::m[I];
+    static_assert(m == 0 || col_minb_listed(m), "a candidate that DNSB_COL_MINB does not list");
     if constexpr (m == 0)
       return k_colpass<R, N, AXIS, FWD>;
     else
@@ -196,8 +197,10 @@ struct Ops {
       if ((e = allow(k_yz<R, N, 0, false>, sm))) return e;
       if ((e = allow(k_yz<R, N, 1, false>, sm))) return e;
       if ((e = allow(k_yz<R, N, 2, false>, sm))) return e;
-      if ((e = allow(k_yz<R, N, 0, true>, sm))) return e;
-      if ((e = allow(k_yz<R, N, 1, true>, sm))) return e;
+      if constexpr (N <= 32) {
+        if ((e = allow(k_yz<R, N, 0, true>, sm))) return e;
+        if ((e = allow(k_yz<R, N, 1, true>, sm))) return e;
+      }
     }
     if constexpr (N > 32) {
       if ((e = allow(k_zstage<R, N, 0>, ZS_SMEM<0>))) return e;
@@ -350,7 +353,7 @@ struct Ops {
     const R invn3 = (R)(1.0 / (double)G.g.nreal);
     if constexpr (HAS_YZ) if (plane(G)) {
       const dim3 grid(N, G.nruns);
-      if constexpr (KIND < 2) {
+      if constexpr (KIND < 2 && N <= 32) {
         if (keep) {
           k_yz<R, N, KIND, true><<<grid, YZ<R, N>::THREADS, YZ<R, N>::SMEM, st>>>(
               work, stale, tw(G), G.g, invn3, keep);
