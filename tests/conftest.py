@@ -15,6 +15,19 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200, sm_100a)")
 
 
+def pytest_collection_modifyitems(items):
+    """Where the reference's own binary is not there, the tests that run it
+    (and fail) come last, so that a run that stops at the first failure has
+    run all the others."""
+    import inspect
+
+    import oracle
+
+    if not os.path.exists(oracle.REF_DNS):
+        names = ("run_ref_dns", "REF_DNS")
+        items.sort(key=lambda it: any(q in inspect.getsource(it.function) for q in names))
+
+
 @pytest.fixture(scope="session")
 def oracle_lib():
     import oracle
