@@ -35,7 +35,7 @@ DNS_FLAG_ENS_PERSISTENT = 4
 SUPPORTED_N = (8, 16, 32, 64, 128, 256, 512)
 KERNELS_PER_STAGE = 6  # passes that dns_time_kernels reports
 KERNELS_PER_STEP = 4 * KERNELS_PER_STAGE
-LAUNCHES_PER_STEP = 16  # kernels: E1, E2 and the next stage's A are one (n <= 32: 8, B, C and D too)
+LAUNCHES_PER_STEP = 16  # of one run with n >= 64: E1, E2 and the next stage's A are one kernel (n <= 32: 8, B, C and D too)
 PASS_NAMES = ("A:x-inverse", "B:y-inverse", "C:z-fused", "D:y-forward", "E1:x-forward", "E2:update")
 
 

@@ -1092,7 +1092,7 @@ static int ens_time_steps(dns_ens *e, float *ms) {
 // The ensemble autotuner: time both schedules on the fresh (all-zero) state,
 // which every step keeps at zero, and keep the faster; the flags can force
 // either.  A persistent schedule exists when every size group is one the
-// persistent kernel compiles (32, 64, 128) and there are at most PMAXG.
+// persistent kernel compiles (64, 128) and there are at most PMAXG.
 static int ens_choose_schedule(dns_ens *e, unsigned flags) {
   const bool can = ens_persistent_supported(e);
   if ((flags & DNS_FLAG_ENS_PERSISTENT) && !can)

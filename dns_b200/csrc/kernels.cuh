@@ -4,20 +4,24 @@
 // and the energy/enstrophy reduction (main.c:257-266).
 //
 // Every kernel is a template on the storage scalar R: double for the FP64
-// path, float for the mixed path (FP32 fields and FFTs; the reductions and
-// the pointwise update arithmetic stay FP64).
+// path, float for the mixed path (FP32 fields, FFTs and pointwise arithmetic;
+// FP64 reductions, and the viscous coefficient nu dt |k|^2 is formed in FP64
+// and rounded once).
 //
 // HBM layout (one "slot" = one complex field on the half spectrum):
 //   spectral slot  [i = kx index][j = ky index][k = kz index], k fastest,
 //                  row pitch nfp = nf rounded up to the column tile width W
 //                  (nf = n/2 + 1; W * sizeof(complex) = 128 bytes), so every
 //                  tile row starts on a 128-byte boundary; the padding
-//                  columns are never read or written.
+//                  columns are never written by a pass and their values never
+//                  used (the FP32 kernels' 16-byte copies of pairs of columns
+//                  read the first of them).
 //   real slot      [x][y][z], z fastest (the .raw layout of main.c:180-185).
 // The same slot shape holds partially transformed data: after the x pass the
 // first index is x instead of kx, after the y pass the second is y.
 //
-// One RK stage = four kernels (two where YZ runs B, C and D in one, n <= 64):
+// One RK stage = four kernels (two where YZ runs B, C and D in one: n <= 32,
+// and three or more runs of n = 64):
 //   B   y backward  5 slots -> u,v,w, omega_z = dv/dx - du/dy, dw/dx, dw/dy
 //   C   z pass      per z line: vorticity from the 6 slots, u and omega to
 //                   real space, N = u x omega, N back to z spectral (stored
@@ -452,11 +456,11 @@ __global__ void __launch_bounds__(ZCfg<N>::THREADS)
 //        z axis being the last, real one); Re y = a, Im y = b.
 //   r2c: Y = a + i b; X_a[k] = (Z[k] + conj Z[N-k]) / 2,
 //        X_b[k] = -i (Z[k] - conj Z[N-k]) / 2.
-// T = N/E threads per line hold E points each.  In the middle stages the
-// pairs (u, omega_y), (w, omega_z), (v, omega_x) read each input slot once
-// and u x omega accumulates in registers; the first and last stages stage
-// the velocity and two partial sums in shared memory (each thread only
-// reads back its own points).
+// T = N/E threads per line hold E points each.  The pairs (u, omega_y), (v,
+// omega_x), (w, omega_z) read each input slot once; what of them waits for the
+// products is in registers or, in FP64 with 16 values per thread, in shared
+// memory (ZC; each thread only reads back its own points).  The first stage
+// transforms the vorticity alone, (omega_x, omega_y) and (omega_z, 0).
 // KIND 0: first stage, velocity from the stale real slots (main.c:344 skips
 //         the back transform at rk == 0); KIND 1: middle stage;
 // KIND 2: last stage, also stores the real velocity as the next stale one.
@@ -1125,7 +1129,9 @@ __global__ void __launch_bounds__(YZ<R, N>::THREADS, YZ<R, N>::MINB)
 //   ST 3:  U_0' = U_3 + ((U_1 - U_0) + 2 (U_2 - U_0) - 2 (U_3 - U_0)) / 3 + dU / 6
 //          (the RK4 sum of main.c:15 written with the stage inputs, which
 //          are kept, in place of an accumulator; the bracket is a sum of
-//          increments, so only the last additions round at |U|)
+//          increments, so it is the roundings at |U| of the stored U_1, U_2
+//          and U_3, weighted by 1/3, 2/3 and 1/3, and the last addition's that
+//          enter, where an accumulator rounds at |U| four times)
 //   x backward of the result: u, v, w and i kx v, i kx w  (TAIL; ST < 0: of
 //   the stored state alone)
 // Outside the 2/3 rule N is masked to zero, so the stage inputs there are the

@@ -409,8 +409,8 @@ struct Ops {
   // Kernel `k` (K_B..K_X) of RK stage `s` for all runs of G, or with s < 0
   // the x transform of the state a step starts from: what it runs, its job
   // table or arguments, and its work items (the launch grid, threads and
-  // shared memory of one block).  The standalone launches (stage_kernel) and
-  // the persistent ensemble kernel's plan are both made from it.
+  // shared memory of one block).  The persistent ensemble kernel's plan is made
+  // from it, and the standalone launches of B and D (stage_kernel).
   static PPhase<R> describe(const Group &G, int s, int k) {
     const Geo &g = G.g;
     PPhase<R> P{};
