@@ -498,8 +498,9 @@ def main() -> int:
     ap.add_argument("--no-n512", action="store_true")
     ap.add_argument("--no-adjoint", action="store_true")
     ap.add_argument("--profile", choices=["fp64", "mixed"], default=None,
-                    help="profiling run: set-up and --warmup steps, then exactly one RK4 "
-                         "step between cudaProfilerStart/Stop (for ncu --profile-from-start off)")
+                    help="profiling run: set-up and --warmup steps, then one dns_step call of two "
+                         "steps between cudaProfilerStart/Stop (for ncu --profile-from-start off); "
+                         "the first of them is in the form that a call repeats")
     args = ap.parse_args()
     world, rank, local = dist_setup()
     if args.impl == "reference":
@@ -518,7 +519,7 @@ def main() -> int:
             c.step(NU, DT, max(1, args.warmup))
             c.synchronize()
             torch.cuda.profiler.start()
-            c.step(NU, DT, 1)
+            c.step(NU, DT, 2)
             c.synchronize()
             torch.cuda.profiler.stop()
             print(json.dumps({"profile": args.profile, "n": args.n, "schedule": c.schedule()}))
