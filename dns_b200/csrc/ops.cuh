@@ -20,7 +20,7 @@ enum { SLOT_SA = 0, SLOT_RK = 3, SLOT_WORK = 7, SLOT_P = 14, NSLOTS = 15 };
 // passes of an RK stage, as dns_time_kernels reports them: A x-inverse, B
 // y-inverse, C z fused, D y-forward, E1 x-forward, E2 pointwise update
 enum { PASSES_PER_STAGE = 6 };
-// the launches that run them: B, C and D (n <= 64: YZ, the three in one), and
+// the launches that run them: B, C and D (or YZ, the three in one: plane()), and
 // X, which is a stage's E1 and E2 and the next stage's A in one kernel
 enum { K_B = 0, K_C = 1, K_D = 2, K_X = 3, K_YZ = 4 };
 
