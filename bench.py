@@ -470,6 +470,12 @@ def adjoint_leg(n: int = 128, snapshots: int = 20):
 def run_reference_arm(args, world, rank):
     if rank != 0:
         return 0
+    import oracle
+
+    if not os.path.exists(oracle.REF_DNS):  # the C restatement is not the reference
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own main.c is not built here "
+                          "(oracle/_ref/dns needs its source)"}), flush=True)
+        return 0
     rate, cores, kind, sample = cpu_reference_rate(args.n)
     line = {
         "impl": "reference", "metric": METRIC if args.n == 256 else METRIC.replace("256^3", f"{args.n}^3"),

@@ -58,3 +58,18 @@ def test_kernel_times_sum_to_the_step():
     kms = np.arange(1.0, 25.0).reshape(4, 6)
     kt = np.array(bench.kernel_times(kms))
     assert kt.shape == (4, 4) and kt.sum() == kms.sum()
+
+
+def test_reference_arm_without_the_reference(monkeypatch, capsys, tmp_path):
+    """Without the reference's binary the arm reports no figure of its own."""
+    import argparse
+    import json
+
+    import bench
+    import oracle
+
+    monkeypatch.setattr(oracle, "REF_DNS", str(tmp_path / "dns"))
+    args = argparse.Namespace(n=16, gpus=1, steps=1, warmup=3)
+    assert bench.run_reference_arm(args, 1, 0) == 0
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "unavailable" in line and "value" not in line
